@@ -29,6 +29,7 @@
 #include <cuda_fp16.h>
 
 #include <cmath>
+#include <numeric>
 
 #include "common.cuh"
 
@@ -37,11 +38,17 @@
 namespace tcb {
 namespace lam {
 
-constexpr int T = 64;
+constexpr int MIN_N = 64;       // smallest grid half-size
+constexpr int TX = 64, TY = 32;  // usfft2d gridding: cells per CTA, 16 x 16 per warp
 constexpr int NT = 256;
-constexpr int CHUNK = NT;
-constexpr int MAXSEG = 4 * CHUNK;
+constexpr int MAXSEG = 4 * NT;   // segments of one search: 4 per thread
 constexpr int EPAD = 8;
+// usfft2d gridding, one staged sample: its value and footprint origin, 9 weights
+// wx and a zero, and 9 weights wy between the zeros that the 16 rows of a warp
+// beside the footprint read (u2_gather)
+constexpr int NSAMP = NT;
+constexpr int XSLOT = 11;             // floats; odd, so that the staging stores spread over the banks
+constexpr int YPAD = 12, YSLOT = 36;  // floats: rows -12 .. 23 from its first, rounded down to 4
 
 // Gridding width/constant exactly as the reference constructors compute them.
 inline void gauss_params(size_t nn, float &mu, int &m) {
@@ -82,6 +89,7 @@ struct U2Geom {
   int ntheta, detw, deth;   // deth = rows of this call (slabs)
   int ntx, nty;             // tiles per axis
   int k, deth0;             // chunk index and full detector height (kv)
+  int pstep;                // order of the angles in u2_gather: p = i pstep mod ntheta
   float wscale;             // PI / sqrt(mu0 mu1 ntheta)
   float c0, c1;             // -PI^2/mu0, -PI^2/mu1
   // sample source
@@ -92,38 +100,62 @@ struct U2Geom {
 };
 
 struct U2Smem {
-  float accr[T][T + 1];  // padded rows: see the fourierrec gridding kernel
-  float acci[T][T + 1];
+  float4 wy[(NSAMP + 1) * YSLOT / 4];  // the last slot stays zero
+  float4 meta[NSAMP + 1];              // value (scaled), tile column of the footprint's first
+                                       // cell, byte offset of tile row 0 in wy (integer bits)
+  float wx[(NSAMP + 1) * XSLOT];
+  unsigned char mask[NSAMP];           // warps whose cells the footprint reaches
   int seg_a[MAXSEG];
   int seg_i0[MAXSEG];
-  int seg_start[MAXSEG + 1];
-  int warp_tot[NT / 32];
+  int seg_start[MAXSEG];
+  int2 warp_tot[NT / 32];
 };
 
-__device__ __forceinline__ int block_exscan(int v, int *warp_tot, int &total) {
+// Packed pair arithmetic: one instruction for two fp32 FMAs.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a,
+                                     unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// Exclusive prefix sums over the block of two values per thread (v becomes the
+// prefix, total the sums).
+__device__ __forceinline__ void block_exscan2(int2 &v, int2 *warp_tot, int2 &total) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int x = v;
+  int2 x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+    const int y0 = __shfl_up_sync(0xffffffffu, x.x, o), y1 = __shfl_up_sync(0xffffffffu, x.y, o);
+    if (lane >= o) {
+      x.x += y0;
+      x.y += y1;
+    }
   }
   if (lane == 31) warp_tot[wid] = x;
   __syncthreads();
-  if (wid == 0) {
-    int t = (lane < NT / 32) ? warp_tot[lane] : 0;
+  int2 base = make_int2(0, 0);
+  total = make_int2(0, 0);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += y;
+  for (int w = 0; w < NT / 32; w++) {
+    const int2 t = warp_tot[w];
+    if (w < wid) {
+      base.x += t.x;
+      base.y += t.y;
     }
-    if (lane < NT / 32) warp_tot[lane] = t;
+    total.x += t.x;
+    total.y += t.y;
   }
-  __syncthreads();
-  int base = wid > 0 ? warp_tot[wid - 1] : 0;
-  total = warp_tot[NT / 32 - 1];
-  __syncthreads();
-  return base + x - v;
+  v.x = base.x + x.x - v.x;
+  v.y = base.y + x.y - v.y;
 }
 
 __device__ __forceinline__ void interval(float c, float a, float b, float &lo, float &hi) {
@@ -131,7 +163,7 @@ __device__ __forceinline__ void interval(float c, float a, float b, float &lo, f
     if (a <= 0.f && 0.f <= b) { lo = -3.0e38f; hi = 3.0e38f; } else { lo = 1.f; hi = -1.f; }
     return;
   }
-  float u0 = a / c, u1 = b / c;
+  const float u0 = __fdividef(a, c), u1 = __fdividef(b, c);
   lo = fminf(u0, u1);
   hi = fmaxf(u0, u1);
 }
@@ -147,8 +179,10 @@ __device__ __forceinline__ void u2_pos(const U2Geom &g, float cphi, float2 csa, 
   float kv = (ty + g.k * g.deth - g.deth0 / 2.0f) / g.deth0;
   x = __fmaf_rn(ku, csa.x, __fmul_rn(__fmul_rn(kv, csa.y), cphi));
   y = __fmaf_rn(-__fmul_rn(kv, csa.x), cphi, __fmul_rn(ku, csa.y));
-  x = (float)fmin(fmax((double)x, -0.5f + 1e-5), 0.5f - 1e-5);
-  y = (float)fmin(fmax((double)y, -0.5f + 1e-5), 0.5f - 1e-5);
+  // take_x clamps in double to +-(0.5 - 1e-5) and rounds: the same floats
+  constexpr float lim = (float)(0.5f - 1e-5);
+  x = fminf(fmaxf(x, -lim), lim);
+  y = fminf(fmaxf(y, -lim), lim);
 }
 
 // Storage of the stage arrays: complex fp32 (float2) or complex fp16
@@ -188,25 +222,54 @@ __device__ __forceinline__ float2 u2_val(const U2Geom &g, const S *__restrict__ 
   return make_float2(v.x * sc, -v.y * sc);
 }
 
+// Adjoint gridding of one slab, output-stationary: a CTA owns 64 x 32 cells of
+// the periodic grid, each warp 16 x 16 of them in registers (lane: one column,
+// 8 rows, real and imaginary), and every sample whose footprint reaches the
+// CTA's cells is staged once in shared memory by one thread.  A warp adds a
+// sample to its 256 cells with four loads (value and origin, the lane's wx, its
+// 8 wy as two 16-byte broadcasts) and 8 packed FMAs; cells outside the
+// footprint read zeros, so no lane branches.  The wy of a slot are laid out by
+// the tile row modulo 4 (12 entries, the outer ones zero), which keeps the
+// 16-byte loads aligned.  The next 256 candidates are located and their values
+// loaded while the current ones are added.  Angles are taken in steps near the
+// golden section, so that the few lines staged together cross different warps'
+// cells and the warps arrive at the barrier together.  Samples are added in one
+// fixed order.
+//
+// Bound: instruction issue, about 26 per warp visit (2.25 visits per sample at
+// 16 x 16 cells) and 8 per staged sample; the packed FMAs alone would take a
+// third of it.  600 angles x 512 samples x 257 slabs on 1024^2 cells: 17.1 ms.
+// One thread per sample adding its 81 cells to a shared-memory tile with atomics
+// took 28.1 ms, 21.8 with this search (the border tiles took every sample of
+// their rows or columns as candidates, eight times the accepted ones).
 template <int M0, int M1, typename S>
-__global__ void __launch_bounds__(NT) u2_gather(const S *__restrict__ src,
-                                                float2 *__restrict__ grid,
-                                                const float2 *__restrict__ cs,
-                                                const float *__restrict__ ex,
-                                                const float *__restrict__ ey, U2Geom geo) {
+__global__ void __launch_bounds__(NT, 3) u2_gather(const S *__restrict__ src,
+                                                   float2 *__restrict__ grid,
+                                                   const float2 *__restrict__ cs,
+                                                   const float *__restrict__ ex,
+                                                   const float *__restrict__ ey, U2Geom geo) {
+  static_assert(M0 == 4 && M1 == 4, "slot layout: 9-cell footprints");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   U2Smem &sm = *reinterpret_cast<U2Smem *>(smem_raw);
   const int n0 = geo.n0, n1 = geo.n1;
   const int ntiles = geo.ntx * geo.nty;
   const int slab = blockIdx.x / ntiles;
   const int tile = blockIdx.x % ntiles;
-  const int ix0 = (tile % geo.ntx) * T, iy0 = (tile / geo.ntx) * T;
-  const int tw = min(T, 2 * n0 - ix0), th = min(T, 2 * n1 - iy0);
+  const int ix0 = (tile % geo.ntx) * TX, iy0 = (tile / geo.ntx) * TY;
+  const int tw = min(TX, 2 * n0 - ix0), th = min(TY, 2 * n1 - iy0);
   const int X0 = ix0 - n0, Y0 = iy0 - n1;
-  for (int k = threadIdx.x; k < T * (T + 1); k += NT) {
-    (&sm.accr[0][0])[k] = 0.f;
-    (&sm.acci[0][0])[k] = 0.f;
-  }
+  const int slot = threadIdx.x, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the warp's cells: columns xw .. xw + 15, rows yw .. yw + 15
+  const int xw = (wid & 3) * 16, yw = (wid >> 2) * 16;
+  const int cx = xw + (lane & 15), cy = yw + (lane >> 4) * 8;
+  const unsigned char *wyc = reinterpret_cast<const unsigned char *>(sm.wy) + 4 * cy;
+  unsigned long long ar[4], ai[4];  // rows (cy, cy + 1), .. of column cx
+#pragma unroll
+  for (int k = 0; k < 4; k++) ar[k] = ai[k] = 0ull;
+  for (int k = threadIdx.x; k < (NSAMP + 1) * YSLOT / 4; k += NT)
+    sm.wy[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = threadIdx.x; k < (NSAMP + 1) * XSLOT; k += NT) sm.wx[k] = 0.f;
+  if (threadIdx.x == 0) sm.meta[NSAMP] = make_float4(0.f, 0.f, 0.f, 0.f);
   int kx_lo = 1, kx_hi = -1, ky_lo = 1, ky_hi = -1;
   for (int k = -1; k <= 1; k++) {
     int lo = X0 - 2 * n0 * k, hi = X0 + tw - 1 - 2 * n0 * k;
@@ -214,41 +277,40 @@ __global__ void __launch_bounds__(NT) u2_gather(const S *__restrict__ src,
     lo = Y0 - 2 * n1 * k; hi = Y0 + th - 1 - 2 * n1 * k;
     if (hi >= -n1 - M1 && lo <= n1 - 1 + M1) { ky_lo = min(ky_lo, k); ky_hi = max(ky_hi, k); }
   }
-  // tiles near the grid border also receive clamped samples: no x (y) pruning there
-  const bool edge_x = (X0 <= -n0 + M0 + 2) || (X0 + tw - 1 >= n0 - 1 - M0 - 2);
-  const bool edge_y = (Y0 <= -n1 + M1 + 2) || (Y0 + th - 1 >= n1 - 1 - M1 - 2);
+  // tiles near the grid border also receive the samples clamped to it: their
+  // range of positions is open on that side (positions stay within +-1)
+  const bool low_x = X0 <= -n0 + M0 + 2, high_x = X0 + tw - 1 >= n0 - 1 - M0 - 2;
+  const bool low_y = Y0 <= -n1 + M1 + 2, high_y = Y0 + th - 1 >= n1 - 1 - M1 - 2;
   const float kv = (slab + geo.k * geo.deth - geo.deth0 / 2.0f) / geo.deth0;
   const int detw = geo.detw;
   const float cphi = cs[geo.ntheta].x;
 
-  for (int pc = 0; pc < geo.ntheta; pc += CHUNK) {
-    int p = pc + threadIdx.x;
-    int my_i0[4], my_len[4], my_img[4];
+  // ranges of positions 2n0 (ku c + ox) in [A-2, B+2], the same along y
+  const float rx = 1.f / (2.f * n0), ry = 1.f / (2.f * n1);
+  const bool single = kx_lo == kx_hi && ky_lo == ky_hi;  // one periodic image
+  const int per = single ? 4 : 1;                        // angles per thread and search
+
+  for (int pc = 0; pc < geo.ntheta; pc += per * NT) {
+    int my_p[4], my_i0[4], my_len[4], my_img[4];
     int nseg = 0, ncand = 0;
-    if (p < geo.ntheta) {
-      float2 csp = cs[p];
-      float ox = kv * csp.y * cphi, oy = -kv * csp.x * cphi;
+    for (int r = 0; r < per; r++) {
+      const int pi = pc + r * NT + threadIdx.x;
+      if (pi >= geo.ntheta) break;
+      const int p = (int)((long long)pi * geo.pstep % geo.ntheta);
+      const float2 csp = cs[p];
+      const float ox = kv * csp.y * cphi, oy = -kv * csp.x * cphi;
       for (int ky = ky_lo; ky <= ky_hi; ky++)
         for (int kx = kx_lo; kx <= kx_hi; kx++) {
-          float lo = -3.0e38f, hi = 3.0e38f, l, h;
-          if (!edge_x) {
-            // 2n0*(ku c + ox) in [A-2, B+2]
-            float a = (float)(X0 - M0 - 2 * n0 * kx - 2) / (2.f * n0) - ox;
-            float b = (float)(X0 + tw - 1 + M0 - 2 * n0 * kx + 2) / (2.f * n0) - ox;
-            interval(csp.x, a, b, l, h);
-            lo = fmaxf(lo, l); hi = fminf(hi, h);
-          } else if (kx != 0) {
-            float a = (float)(X0 - M0 - 2 * n0 * kx - 2) / (2.f * n0) - ox;
-            float b = (float)(X0 + tw - 1 + M0 - 2 * n0 * kx + 2) / (2.f * n0) - ox;
-            interval(csp.x, a, b, l, h);
-            lo = fmaxf(lo, l); hi = fminf(hi, h);
-          }
-          if (!edge_y || ky != 0) {
-            float a = (float)(Y0 - M1 - 2 * n1 * ky - 2) / (2.f * n1) - oy;
-            float b = (float)(Y0 + th - 1 + M1 - 2 * n1 * ky + 2) / (2.f * n1) - oy;
-            interval(csp.y, a, b, l, h);
-            lo = fmaxf(lo, l); hi = fminf(hi, h);
-          }
+          const bool ax = kx == 0 ? low_x : kx == 1, bx = kx == 0 ? high_x : kx == -1;
+          const bool ay = ky == 0 ? low_y : ky == 1, by = ky == 0 ? high_y : ky == -1;
+          const int ex0 = X0 - 2 * n0 * kx, ey0 = Y0 - 2 * n1 * ky;
+          float lo, hi, l, h;
+          interval(csp.x, (ax ? -1.f : (float)(ex0 - M0 - 2) * rx) - ox,
+                   (bx ? 1.f : (float)(ex0 + tw + M0 + 1) * rx) - ox, lo, hi);
+          interval(csp.y, (ay ? -1.f : (float)(ey0 - M1 - 2) * ry) - oy,
+                   (by ? 1.f : (float)(ey0 + th + M1 + 1) * ry) - oy, l, h);
+          lo = fmaxf(lo, l);
+          hi = fminf(hi, h);
           if (lo > hi) continue;
           lo = fmaxf(lo, -1.f);
           hi = fminf(hi, 1.f);
@@ -256,6 +318,7 @@ __global__ void __launch_bounds__(NT) u2_gather(const S *__restrict__ src,
           int i0 = max(0, (int)floorf(lo * detw + detw * 0.5f) - 1);
           int i1 = min(detw - 1, (int)ceilf(hi * detw + detw * 0.5f) + 1);
           if (i1 < i0) continue;
+          my_p[nseg] = p;
           my_i0[nseg] = i0;
           my_len[nseg] = i1 - i0 + 1;
           my_img[nseg] = (kx + 1) + 3 * (ky + 1);
@@ -263,73 +326,141 @@ __global__ void __launch_bounds__(NT) u2_gather(const S *__restrict__ src,
           nseg++;
         }
     }
-    int seg_total, cand_total;
-    int seg_off = block_exscan(nseg, sm.warp_tot, seg_total);
-    int cand_off = block_exscan(ncand, sm.warp_tot, cand_total);
-    if (cand_total == 0) continue;
+    int2 off = make_int2(nseg, ncand), tot;
+    block_exscan2(off, sm.warp_tot, tot);
+    const int seg_total = tot.x, cand_total = tot.y;
     {
-      int c = cand_off;
+      int c = off.y;
       for (int k = 0; k < nseg; k++) {
-        sm.seg_a[seg_off + k] = p | (my_img[k] << 20);
-        sm.seg_i0[seg_off + k] = my_i0[k];
-        sm.seg_start[seg_off + k] = c;
+        sm.seg_a[off.x + k] = my_p[k] | (my_img[k] << 20);
+        sm.seg_i0[off.x + k] = my_i0[k];
+        sm.seg_start[off.x + k] = c;
         c += my_len[k];
       }
     }
     __syncthreads();
-    for (int j = threadIdx.x; j < cand_total; j += NT) {
-      int lo = 0, hi = seg_total - 1;
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (sm.seg_start[mid] <= j) lo = mid; else hi = mid - 1;
+    // candidate j0 + slot: its value and where its footprint lies in the tile
+    float px = 0.f, py = 0.f;
+    float2 gv = make_float2(0.f, 0.f);
+    int b0 = 0, b1 = 0, lx0 = 0, ly0 = 0, mask = 0;
+    auto locate = [&](int j0) {
+      mask = 0;
+      const int jw = j0 + wid * 32, j = jw + lane;
+      if (jw >= cand_total) return;
+      // the segment of the warp's first candidate by two ballots, then onwards
+      int q = lane * 32;
+      const int blk = __popc(__ballot_sync(0xffffffffu, q < seg_total && sm.seg_start[q] <= jw)) - 1;
+      q = blk * 32 + lane;
+      int sg = blk * 32 - 1 +
+               __popc(__ballot_sync(0xffffffffu, q < seg_total && sm.seg_start[q] <= jw));
+      if (j >= cand_total) return;
+      while (sg + 1 < seg_total && sm.seg_start[sg + 1] <= j) sg++;
+      const int a = sm.seg_a[sg];
+      const int img = a >> 20, ang = a & 0xFFFFF;
+      const int tx = sm.seg_i0[sg] + (j - sm.seg_start[sg]);
+      u2_pos(geo, cphi, cs[ang], tx, slab, px, py);
+      b0 = (int)floorf(2 * n0 * px) - M0;
+      b1 = (int)floorf(2 * n1 * py) - M1;
+      lx0 = b0 + 2 * n0 * (img % 3 - 1) - X0;
+      ly0 = b1 + 2 * n1 * (img / 3 - 1) - Y0;
+      if (lx0 > tw - 1 || lx0 + 2 * M0 < 0 || ly0 > th - 1 || ly0 + 2 * M1 < 0) return;
+      // warps of the columns 16 k .. and rows 16 k .. the footprint reaches
+      int mx = (2 << (min(lx0 + 2 * M0, TX - 1) >> 4)) - (1 << (max(lx0, 0) >> 4));
+      if (ly0 <= 15) mask |= mx;
+      if (ly0 + 2 * M1 >= 16) mask |= mx << 4;
+      gv = u2_val(geo, src, tx, slab, ang);
+    };
+    locate(0);
+    for (int j0 = 0; j0 < cand_total; j0 += NSAMP) {
+      __syncthreads();  // the slots are free
+      sm.mask[slot] = (unsigned char)mask;
+      if (mask) {
+        sm.meta[slot] = make_float4(gv.x * geo.wscale, gv.y * geo.wscale, __int_as_float(lx0),
+                                    __int_as_float(4 * (slot * YSLOT + YPAD - (ly0 & ~3))));
+        float *o = sm.wx + slot * XSLOT;
+#pragma unroll
+        for (int t = 0; t < 2 * M0 + 1; t++) {
+          const float w0 = ex[b0 + t + n0 + M0 + EPAD] - px;
+          o[t] = __expf(geo.c0 * (w0 * w0));
+        }
+        float w[2 * M1 + 1];
+#pragma unroll
+        for (int t = 0; t < 2 * M1 + 1; t++) {
+          const float w1 = ey[b1 + t + n1 + M1 + EPAD] - py;
+          w[t] = __expf(geo.c1 * (w1 * w1));
+        }
+        const int sh = ly0 & 3;
+        float v[12];
+#pragma unroll
+        for (int e = 0; e < 12; e++) {
+          float r = 0.f;
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+            if (e - q >= 0 && e - q <= 2 * M1 && sh == q) r = w[e - q];
+          v[e] = r;
+        }
+        float4 *oy = sm.wy + (slot * YSLOT + YPAD) / 4;
+#pragma unroll
+        for (int e = 0; e < 3; e++)
+          oy[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
       }
-      int a = sm.seg_a[lo];
-      int img = a >> 20, ang = a & 0xFFFFF;
-      int tx = sm.seg_i0[lo] + (j - sm.seg_start[lo]);
-      float x0, y0;
-      u2_pos(geo, cphi, cs[ang], tx, slab, x0, y0);
-      int b0 = (int)floorf(2 * n0 * x0) - M0;
-      int b1 = (int)floorf(2 * n1 * y0) - M1;
-      int kx = img % 3 - 1, ky = img / 3 - 1;
-      int lx0 = b0 + 2 * n0 * kx - X0;
-      int ly0 = b1 + 2 * n1 * ky - Y0;
-      if (lx0 > tw - 1 || lx0 + 2 * M0 < 0 || ly0 > th - 1 || ly0 + 2 * M1 < 0) continue;
-      float2 gv = u2_val(geo, src, tx, slab, ang);
-      float k0[2 * M0 + 1], k1[2 * M1 + 1];
-#pragma unroll
-      for (int t = 0; t < 2 * M0 + 1; t++) {
-        float w0 = ex[b0 + t + n0 + M0 + EPAD] - x0;
-        k0[t] = __expf(geo.c0 * (w0 * w0));
-      }
-#pragma unroll
-      for (int t = 0; t < 2 * M1 + 1; t++) {
-        float w1 = ey[b1 + t + n1 + M1 + EPAD] - y0;
-        k1[t] = __expf(geo.c1 * (w1 * w1));
-      }
-      float gx = gv.x * geo.wscale, gy = gv.y * geo.wscale;
-#pragma unroll
-      for (int t1 = 0; t1 < 2 * M1 + 1; t1++) {
-        int ly = ly0 + t1;
-        if (ly < 0 || ly >= th) continue;
-#pragma unroll
-        for (int t0 = 0; t0 < 2 * M0 + 1; t0++) {
-          int lx = lx0 + t0;
-          if (lx < 0 || lx >= tw) continue;
-          float w = k0[t0] * k1[t1];
-          atomicAdd(&sm.accr[ly][lx], w * gx);
-          atomicAdd(&sm.acci[ly][lx], w * gy);
+      __syncthreads();
+      locate(j0 + NSAMP);
+      for (int c0 = 0; c0 < NSAMP; c0 += 32) {
+        unsigned bits = __ballot_sync(0xffffffffu, (sm.mask[c0 + lane] >> wid) & 1);
+        while (bits) {
+          // two samples at a time, the zero slot for a missing second
+          const int s0 = c0 + __ffs(bits) - 1;
+          bits &= bits - 1;
+          const int s1 = bits ? c0 + __ffs(bits) - 1 : NSAMP;
+          bits &= bits - 1;
+          const float4 ma = sm.meta[s0], mb = sm.meta[s1];
+          const int ya = __float_as_int(ma.w),
+                    yb = s1 < NSAMP ? __float_as_int(mb.w) : 4 * (NSAMP * YSLOT - yw);
+          const unsigned da = min((unsigned)(cx - __float_as_int(ma.z)), 9u);
+          const unsigned db = min((unsigned)(cx - __float_as_int(mb.z)), 9u);
+          const float xa = sm.wx[s0 * XSLOT + da], xb = sm.wx[s1 * XSLOT + db];
+          const ulonglong2 *wa = reinterpret_cast<const ulonglong2 *>(wyc + ya);
+          const ulonglong2 *wb = reinterpret_cast<const ulonglong2 *>(wyc + yb);
+          const ulonglong2 a0 = wa[0], a1 = wa[1], q0 = wb[0], q1 = wb[1];
+          float gr = xa * ma.x, gi = xa * ma.y;
+          unsigned long long r = pack2(gr, gr), i = pack2(gi, gi);
+          fma2(ar[0], a0.x, r);
+          fma2(ai[0], a0.x, i);
+          fma2(ar[1], a0.y, r);
+          fma2(ai[1], a0.y, i);
+          fma2(ar[2], a1.x, r);
+          fma2(ai[2], a1.x, i);
+          fma2(ar[3], a1.y, r);
+          fma2(ai[3], a1.y, i);
+          gr = xb * mb.x;
+          gi = xb * mb.y;
+          r = pack2(gr, gr);
+          i = pack2(gi, gi);
+          fma2(ar[0], q0.x, r);
+          fma2(ai[0], q0.x, i);
+          fma2(ar[1], q0.y, r);
+          fma2(ai[1], q0.y, i);
+          fma2(ar[2], q1.x, r);
+          fma2(ai[2], q1.x, i);
+          fma2(ar[3], q1.y, r);
+          fma2(ai[3], q1.y, i);
         }
       }
     }
-    __syncthreads();
+    __syncthreads();  // the segment list is rewritten for the next angles
   }
   float2 *gz = grid + (size_t)slab * (2 * n0) * (2 * n1);
-  for (int k = threadIdx.x; k < T * T; k += NT) {
-    int ly = k / T, lx = k % T;
-    if (ly >= th || lx >= tw) continue;
-    int ix = ix0 + lx, iy = iy0 + ly;
-    float s = (float)(sgn_idx(ix + M0) * sgn_idx(iy + M1));
-    gz[(size_t)iy * (2 * n0) + ix] = make_float2(sm.accr[ly][lx] * s, sm.acci[ly][lx] * s);
+  const int ix = ix0 + cx;
+  if (cx >= tw) return;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float2 re = unpack2(ar[k]), im = unpack2(ai[k]);
+    const int iy = iy0 + cy + 2 * k;  // 2 n1 is even: both rows are inside or neither is
+    if (iy >= 2 * n1) break;
+    const float s = (float)(sgn_idx(ix + M0) * sgn_idx(iy + M1));
+    gz[(size_t)iy * (2 * n0) + ix] = make_float2(re.x * s, im.x * s);
+    gz[(size_t)(iy + 1) * (2 * n0) + ix] = make_float2(-re.y * s, -im.y * s);
   }
 }
 
@@ -712,8 +843,8 @@ extern "C" int tcb_usfft2d_create(tcb_usfft2d **out, size_t n0_, size_t n1_, siz
   *out = nullptr;
   // argument order of cfunc_usfft2d: (n0, n1, n2) from Python = (slabs, y, x)
   size_t n0 = n2_, n1 = n1_, n2 = n0_;
-  TCB_CHECK_ARG(n0 >= (size_t)T && n1 >= (size_t)T && n0 % 2 == 0 && n1 % 2 == 0,
-                "tcb_usfft2d_create: grid sizes must be even and >= %d", T);
+  TCB_CHECK_ARG(n0 >= (size_t)MIN_N && n1 >= (size_t)MIN_N && n0 % 2 == 0 && n1 % 2 == 0,
+                "tcb_usfft2d_create: grid sizes must be even and >= %d", MIN_N);
   TCB_CHECK_ARG(n2 >= 1 && ntheta >= 1 && ntheta < (1u << 20) && detw >= 2 && deth >= 1,
                 "tcb_usfft2d_create: bad sizes");
   float mu0, mu1;
@@ -732,11 +863,14 @@ extern "C" int tcb_usfft2d_create(tcb_usfft2d **out, size_t n0_, size_t n1_, siz
   g.ntheta = (int)ntheta;
   g.detw = (int)detw;
   g.deth = (int)deth;
-  g.ntx = (int)ceil_div(2 * n0, T);
-  g.nty = (int)ceil_div(2 * n1, T);
+  g.ntx = (int)ceil_div(2 * n0, TX);
+  g.nty = (int)ceil_div(2 * n1, TY);
   g.wscale = (float)(LAM_PI_D / sqrtf(mu0 * mu1 * ntheta));
   g.c0 = (float)(-LAM_PI_D * LAM_PI_D / mu0);
   g.c1 = (float)(-LAM_PI_D * LAM_PI_D / mu1);
+  // a step near the golden section of ntheta and prime to it
+  g.pstep = (int)(0.381966 * ntheta) + 1;
+  while (std::gcd((size_t)g.pstep, ntheta) != 1) g.pstep++;
   h->n2 = n2;
   auto fail = [&](int code, const char *what) {
     set_error("tcb_usfft2d_create: %s", what);
