@@ -9,20 +9,19 @@
 //  * ifftshiftc before/after the 1D FFT becomes an index shift by n/2 plus a
 //    (-1)^k sign at read time, so g is transformed in a single cuFFT call.
 //  * Gridding is output-stationary and atomic-free.  The periodic (2n)^2 grid
-//    is cut into 32x16-cell tiles; each warp of a tile's CTA owns one 8x4
-//    block of cells (one cell per lane) and keeps the accumulators of up to
-//    16 slice pairs in registers.  The polar samples whose (2m+1)^2 footprint
-//    reaches a tile, and for each 8x4 block the subset reaching it, depend on
-//    the angles only; they are listed once when the object is created (theta
-//    is fixed for the object's lifetime, as in the reference).  Per launch a
-//    CTA stages the spectrum values of its samples (all pairs, pair-innermost)
-//    in shared memory, and every lane adds w(cell, sample) * g[pair] for the
-//    samples of its block: two exp per lane per sample serve all pairs.
+//    is cut into 32x16-cell tiles; the warps of a tile's CTA own 8x8 cells each
+//    and keep the accumulators of up to 8 slice pairs in registers.  The polar
+//    samples whose (2m+1)^2 footprint reaches a tile depend on the angles only;
+//    they are listed once when the object is created (theta is fixed for the
+//    object's lifetime, as in the reference).  Per launch a CTA stages the
+//    separable weights and the spectrum values (all pairs, pair-innermost) of
+//    its samples in shared memory, and every lane adds w(cell, sample) * g[pair]
+//    for the samples that reach its warp's cells (grid_regs).
 //    There is no memset, no wrap pass (the grid is periodic by
 //    construction), no global atomics, the summation order is fixed (results
 //    are bit-reproducible) and the fftshift sign before the 2D FFT is
-//    applied in the store.  Tiles are dispatched centre-first because the
-//    polar sample density peaks at the origin.
+//    applied in the store.  The polar sample density peaks at the origin, so
+//    long tiles are split into several work items, dispatched longest first.
 //  * The 2D FFT runs on a dense (2n)^2 grid; the fftshift after it, divphi,
 //    circ and (optionally) the real/imaginary unpacking of the slice pairs
 //    are one kernel.
@@ -34,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <numeric>
 #include <vector>
 
 #include "common.cuh"
@@ -47,11 +47,6 @@ namespace fr {
 
 constexpr int M = 4;            // gridding half-width for eps = 1e-3 (any n)
 constexpr int TX = 32, TY = 16; // grid tile (cells)
-constexpr int RX = 8, RY = 4;   // cell block owned by one warp (one cell per lane)
-constexpr int NRX = TX / RX, NRY = TY / RY;
-constexpr int NREG = NRX * NRY; // 16 blocks = 16 warps per tile
-constexpr int NTH = NREG * 32;  // 512 threads
-constexpr int SC = 256;         // samples staged per chunk
 constexpr int SETUP_NT = 256;
 // Margin of the ell/(2n) table: __cosf/__sinf may exceed 1 in magnitude by an
 // ulp, which moves floor(2n*x0) one cell below -n.
@@ -160,13 +155,14 @@ __device__ __forceinline__ bool local_range(int f, int origin, int width, int tw
 
 // ---- per-geometry sample lists ------------------------------------------
 // pass 0: count the samples whose footprint reaches each tile;
-// pass 1: write them (packed p*n+i) in angle-then-radius order.
+// pass 1: write them (packed p*n+i) in angle-then-radius order, the angles in
+// the order p = k pstep mod nproj.
 // Tiles of TXT x TYT cells (ntx = ceil(2n / TXT) per row).
 template <int TXT, int TYT>
 __global__ void __launch_bounds__(SETUP_NT)
     list_tile_samples(const float2 *__restrict__ cs, const float *__restrict__ rtab, Geom geo,
-                      int pass, int *__restrict__ counts, const long long *__restrict__ offs,
-                      int *__restrict__ list) {
+                      int pstep, int pass, int *__restrict__ counts,
+                      const long long *__restrict__ offs, int *__restrict__ list) {
   __shared__ int warp_tot[SETUP_NT / 32];
   const int n = geo.n, twon = geo.twon, nproj = geo.nproj;
   const int tile = blockIdx.x;
@@ -185,7 +181,8 @@ __global__ void __launch_bounds__(SETUP_NT)
   long long base = pass ? offs[tile] : 0;
   int running = 0;
   for (int pc = 0; pc < nproj; pc += SETUP_NT) {
-    int p = pc + threadIdx.x;
+    const int pi = pc + threadIdx.x;
+    const int p = pi < nproj ? (int)((long long)pi * pstep % nproj) : nproj;
     int cnt = 0;
     int i0s[4], i1s[4], ks[4];
     int nr = 0;
@@ -241,83 +238,54 @@ __global__ void __launch_bounds__(SETUP_NT)
   if (!pass && threadIdx.x == 0) counts[tile] = running;
 }
 
-// pass 0: count, for each 8x4 block of each tile, the tile samples reaching
-// it; pass 1: write their tile-local indices (ascending).
-__global__ void __launch_bounds__(NTH)
-    list_block_samples(const float2 *__restrict__ cs, const float *__restrict__ rtab, Geom geo,
-                       const long long *__restrict__ toffs, const int *__restrict__ tlist,
-                       int pass, int *__restrict__ counts, const long long *__restrict__ boffs,
-                       int *__restrict__ blist) {
-  __shared__ int wcnt[NREG][NTH / 32];
-  __shared__ int run[NREG];
-  const int n = geo.n, twon = geo.twon;
-  const int tile = blockIdx.x;
-  const int ix0 = (tile % geo.ntx) * TX, iy0 = (tile / geo.ntx) * TY;
-  const int tw = min(TX, twon - ix0), th = min(TY, twon - iy0);
-  const int X0 = ix0 - n, Y0 = iy0 - n;
-  const float twonf = (float)(2 * n);
-  const long long t0 = toffs[tile];
-  const int S = (int)(toffs[tile + 1] - t0);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x < NREG) run[threadIdx.x] = 0;
-  __syncthreads();
-  for (int base = 0; base < S; base += NTH) {
-    int k = base + threadIdx.x;
-    unsigned mask = 0;
-    if (k < S) {
-      int s = tlist[t0 + k];
-      int p = s / n, i = s % n;
-      float x0, y0;
-      int fx, fy, xa, xb, ya, yb;
-      sample_pos(cs, rtab, p, i, twonf, x0, y0, fx, fy);
-      if (local_range(fx, X0, tw, twon, xa, xb) && local_range(fy, Y0, th, twon, ya, yb)) {
-        for (int ry = ya / RY; ry <= yb / RY; ry++)
-          for (int rx = xa / RX; rx <= xb / RX; rx++) mask |= 1u << (ry * NRX + rx);
-      }
-    }
-    unsigned ballots[NREG];
-#pragma unroll
-    for (int r = 0; r < NREG; r++) {
-      ballots[r] = __ballot_sync(0xffffffffu, (mask >> r) & 1u);
-      if (lane == 0) wcnt[r][wid] = __popc(ballots[r]);
-    }
-    __syncthreads();
-    if (threadIdx.x < NREG) {  // exclusive offsets of each warp within this chunk
-      int r = threadIdx.x, acc = run[r];
-      for (int w = 0; w < NTH / 32; w++) {
-        int c = wcnt[r][w];
-        wcnt[r][w] = acc;
-        acc += c;
-      }
-      run[r] = acc;
-    }
-    __syncthreads();
-    if (pass) {
-      unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-      for (int r = 0; r < NREG; r++)
-        if ((mask >> r) & 1u)
-          blist[boffs[tile * NREG + r] + wcnt[r][wid] + __popc(ballots[r] & lt)] = k;
-    }
-    __syncthreads();
-  }
-  if (!pass && threadIdx.x < NREG) counts[tile * NREG + threadIdx.x] = run[threadIdx.x];
-}
-
 // ---- gridding --------------------------------------------------------------
 // G: [nz, nproj, n] complex, plain forward FFT of each projection.
 // grid: [nz, 2n, 2n] complex (fftshift sign included).
-constexpr int KREC = 2 + 2 * (2 * M + 2);  // staged record: origin + 10 x-weights + 10 y-weights
+// Work is dealt out in items: up to item_len listed samples of one tile
+// (item_len: 1024, or an eighth of a CTA slot's share of all samples if that
+// is more).  The polar samples crowd the grid centre -- at 1024 x 720 the
+// centre tile lists 50 times the mean -- so whole tiles per CTA would leave
+// the chip waiting for a few; a split tile's partial sums go to a workspace
+// and grid_combine adds them in order.
+struct GridItem {
+  int tile, first, count;  // samples first .. first + count - 1 of the tile's list
+  int part;                // workspace slot of a split tile, -1: store to the grid
+};
+struct GridSplit {
+  int tile, part, nparts;  // workspace slots part .. part + nparts - 1
+};
+
+constexpr int GT = 256;                    // threads: 8 warps of 8 x 8 cells per tile
+constexpr int GS = GT;                     // samples staged at a time, one per thread
+constexpr int GXPAD = 7, GXSLOT = 23;      // x-weights of cells -7 .. 15 from the footprint's first
+constexpr int GYPAD = 6, GYSLOT = 22;      // y-weights of cells -6 .. 15 from its first, rounded down to 2
+static_assert(TX == 32 && TY == 16, "8 warps of 8 x 8 cells");
+
 template <int Z>
 struct GridSmem {
-  float4 g[Z / 2][SC];  // (g_z.x, g_z.y, g_z+1.x, g_z+1.y) of each staged sample
-  // per staged sample: [0] tile-local footprint origin (lx0 | ly0 << 16),
-  // [2..11] x-weights exp(c1 (ell/2n - x0)^2) for the 9 footprint columns and
-  // a trailing 0, [12..21] the same along y.  A lane reads the weight of its
-  // own column/row, so the exps are computed once per staged sample instead
-  // of once per lane.
-  int rec[SC][KREC];
+  // values of one sample, padded so that the staging stores spread over the banks
+  static constexpr int GSTR = Z / 2 + 1 - Z / 2 % 2;
+  float4 g[(GS + 1) * GSTR];
+  float2 wy[(GS + 1) * GYSLOT / 2 + 1];
+  float wx[(GS + 1) * GXSLOT];
+  int2 base[GS + 1];           // where the tile's cell (0, 0) lies in the weight slots
+  unsigned char mask[GS];      // warps whose cells the footprint reaches
 };
+
+__device__ __forceinline__ unsigned long long dup2(float a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a,
+                                     unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
 
 // Footprint origin relative to the tile on a periodic axis, in [-2M, twon-2M-1].
 __device__ __forceinline__ int tile_origin(int f, int origin, int twon) {
@@ -328,120 +296,186 @@ __device__ __forceinline__ int tile_origin(int f, int origin, int twon) {
   return t;
 }
 
+// fp32 gridding of Z slice pairs.  Each of a CTA's 8 warps owns 8 x 8 cells of
+// the 32 x 16 tile, two rows of one column per lane, every pair's real and
+// imaginary sums in registers.  256 samples at a time are staged in shared
+// memory, one per thread: 9 x-weights and 9 y-weights, each between zeros that
+// the cells of a reached warp outside the footprint read (so no lane branches),
+// and the Z values.  Per sample and warp a lane forms its two weights once and
+// adds them times every pair's value with packed FMAs (broadcast 16-byte
+// loads); the next 256 samples are located and their values loaded meanwhile.
+// Sums run in the list's order.
+//
+// Bound: instruction issue; the FP32 pipe alone would take 4 cell sums per
+// useful one ((8 + 8)^2 cells of 8 x 8 blocks reach a sample).  8 x 8 cells per
+// warp cost 16 + 6 / Z lane-FMAs per pair and sample against 36 at 16 x 16;
+// 8 x 4 (12) spend it again on loading the values.  8 pairs: 0.10 ms at 512 x
+// 360, 0.29 ms at 1024 x 720, 1.15 ms at 2048 x 1500; one cell per lane, samples
+// sorted into 8 x 4 blocks and whole tiles per CTA took 0.65 ms at 1024 x 720.
 template <int Z>
-__global__ void __launch_bounds__(NTH, 2)
-    grid_blocks(const float2 *__restrict__ G, float2 *__restrict__ grid,
-                const float2 *__restrict__ cs, const float *__restrict__ rtab,
-                const float *__restrict__ etab, const int *__restrict__ tile_order,
-                const long long *__restrict__ toffs, const int *__restrict__ tlist,
-                const long long *__restrict__ boffs, const int *__restrict__ blist, Geom geo) {
+__global__ void __launch_bounds__(GT, 3)
+    grid_regs(const float2 *__restrict__ G, float2 *__restrict__ grid,
+              float2 *__restrict__ parts, const float2 *__restrict__ cs,
+              const float *__restrict__ rtab, const float *__restrict__ etab,
+              const GridItem *__restrict__ items, const long long *__restrict__ toffs,
+              const int *__restrict__ tlist, Geom geo) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GridSmem<Z> &sm = *reinterpret_cast<GridSmem<Z> *>(smem_raw);
+  constexpr int GSTR = GridSmem<Z>::GSTR;
   const int n = geo.n, twon = geo.twon, nproj = geo.nproj;
   const int zgroups = (geo.nz + Z - 1) / Z;
-  const int tile = tile_order[blockIdx.x / zgroups];
+  const GridItem item = items[blockIdx.x / zgroups];
   const int z0 = (blockIdx.x % zgroups) * Z;
-  const int ix0 = (tile % geo.ntx) * TX, iy0 = (tile / geo.ntx) * TY;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  // this lane's cell, tile-local and global
-  const int lx = (wid % NRX) * RX + (lane % RX);
-  const int ly = (wid / NRX) * RY + (lane / RX);
-  const int cx = ix0 + lx, cy = iy0 + ly;
+  const int ix0 = (item.tile % geo.ntx) * TX, iy0 = (item.tile / geo.ntx) * TY;
+  const int slot = threadIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int xw = (wid & 3) * 8, yw = (wid >> 2) * 8;
+  const int lx = xw + (lane & 7), ly = yw + 2 * (lane >> 3);  // cells (lx, ly), (lx, ly + 1)
   const int X0 = ix0 - n, Y0 = iy0 - n;
   const float twonf = (float)(2 * n);
-  const int half = n / 2;
-  float ar[Z], ai[Z];
+  unsigned long long a0[Z], a1[Z];  // (re, im) of the two cells
 #pragma unroll
-  for (int z = 0; z < Z; z++) ar[z] = ai[z] = 0.f;
+  for (int z = 0; z < Z; z++) a0[z] = a1[z] = 0ull;
+  for (int k = threadIdx.x; k < (GS + 1) * GXSLOT; k += GT) sm.wx[k] = 0.f;
+  for (int k = threadIdx.x; k < (GS + 1) * GYSLOT / 2 + 1; k += GT) sm.wy[k] = make_float2(0.f, 0.f);
+  if (threadIdx.x < GSTR) sm.g[GS * GSTR + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int *list = tlist + toffs[item.tile] + item.first;
 
-  const long long t0 = toffs[tile];
-  const int S = (int)(toffs[tile + 1] - t0);
-  long long bcur = boffs[tile * NREG + wid];
-  const long long bend = boffs[tile * NREG + wid + 1];
-
-  for (int c0 = 0; c0 < S; c0 += SC) {
-    const int cnt = min(SC, S - c0);
-    // stage footprint origins and separable weights
-    for (int k = threadIdx.x; k < cnt; k += NTH) {
-      int s = tlist[t0 + c0 + k];
-      int p = s / n, i = s % n;
-      float x0, y0;
-      int fx, fy;
-      sample_pos(cs, rtab, p, i, twonf, x0, y0, fx, fy);
-      int *r = sm.rec[k];
-      r[0] = (tile_origin(fx, X0, twon) & 0xFFFF) | (tile_origin(fy, Y0, twon) << 16);
-      r[1] = 0;
+  float x0 = 0.f, y0 = 0.f;
+  int fx = 0, fy = 0, lx0 = 0, ly0 = 0, mask = 0;
+  float2 v[Z];
+  auto locate = [&](int c0) {
+    mask = 0;
+    const int k = c0 + slot;
+    if (k >= item.count) return;
+    const int s = __ldg(list + k);
+    const int p = s / n, i = s - p * n;
+    sample_pos(cs, rtab, p, i, twonf, x0, y0, fx, fy);
+    lx0 = tile_origin(fx, X0, twon);
+    ly0 = tile_origin(fy, Y0, twon);
+    // warps of the columns 8 k .. and rows 8 k .. the footprint reaches
+    const int mx = (2 << (min(lx0 + 2 * M, TX - 1) >> 3)) - (1 << (max(lx0, 0) >> 3));
+    if (ly0 <= 7) mask |= mx;
+    if (ly0 + 2 * M >= 8) mask |= mx << 4;
+    int ii = i + n / 2;
+    if (ii >= n) ii -= n;
+    const float sg = (i & 1) ? -geo.scale : geo.scale;
+    const float2 *src = G + ((size_t)z0 * nproj + p) * n + ii;
+    const size_t pair = (size_t)nproj * n;
+#pragma unroll
+    for (int z = 0; z < Z; z++) {
+      v[z] = make_float2(0.f, 0.f);
+      if (z0 + z < geo.nz) {
+        v[z] = __ldg(src + z * pair);
+        v[z].x *= sg;
+        v[z].y *= sg;
+      }
+    }
+  };
+  locate(0);
+  for (int c0 = 0; c0 < item.count; c0 += GS) {
+    __syncthreads();  // the slots are free
+    sm.mask[slot] = (unsigned char)mask;
+    if (mask) {
+      sm.base[slot] = make_int2(slot * GXSLOT + GXPAD - lx0, slot * GYSLOT + GYPAD - (ly0 & ~1));
+      float w[2 * M + 3];  // 9 weights between zeros
+      w[0] = w[2 * M + 2] = 0.f;
+      float *ox = sm.wx + slot * GXSLOT + GXPAD;
 #pragma unroll
       for (int d = 0; d < 2 * M + 1; d++) {
-        float w0 = etab[fx - M + d + n + M + EPAD] - x0;
-        float w1 = etab[fy - M + d + n + M + EPAD] - y0;
-        r[2 + d] = __float_as_int(__expf(geo.coeff1 * w0 * w0));
-        r[2 + 2 * M + 2 + d] = __float_as_int(__expf(geo.coeff1 * w1 * w1));
+        const float w0 = etab[fx - M + d + n + M + EPAD] - x0;
+        const float w1 = etab[fy - M + d + n + M + EPAD] - y0;
+        ox[d] = __expf(geo.coeff1 * w0 * w0);
+        w[1 + d] = __expf(geo.coeff1 * w1 * w1);
       }
-      r[2 + 2 * M + 1] = 0;
-      r[2 + 2 * (2 * M + 1) + 1] = 0;
-    }
-    // stage spectrum values of Z pairs, pair-innermost; consecutive threads
-    // read consecutive samples of one pair (coalesced along the radius)
-    for (int e = threadIdx.x; e < cnt * (Z / 2); e += NTH) {
-      int k = e % cnt, zp = e / cnt;
-      int s = tlist[t0 + c0 + k];
-      int p = s / n, i = s % n;
-      int ii = i + half;
-      if (ii >= n) ii -= n;
-      float sg = (i & 1) ? -geo.scale : geo.scale;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      int za = z0 + 2 * zp, zb = za + 1;
-      if (za < geo.nz) {
-        float2 a = G[((size_t)za * nproj + p) * n + ii];
-        v.x = a.x * sg;
-        v.y = a.y * sg;
-      }
-      if (zb < geo.nz) {
-        float2 b = G[((size_t)zb * nproj + p) * n + ii];
-        v.z = b.x * sg;
-        v.w = b.y * sg;
-      }
-      sm.g[zp][k] = v;
+      float2 *oy = sm.wy + (slot * GYSLOT + GYPAD) / 2;
+      const bool odd = ly0 & 1;
+#pragma unroll
+      for (int e = 0; e < M + 1; e++)
+        oy[e] = odd ? make_float2(w[2 * e], w[2 * e + 1]) : make_float2(w[2 * e + 1], w[2 * e + 2]);
+#pragma unroll
+      for (int z = 0; z < Z; z += 2)
+        sm.g[slot * GSTR + z / 2] = make_float4(v[z].x, v[z].y, v[z + 1].x, v[z + 1].y);
     }
     __syncthreads();
-    // this warp's samples within the chunk (block list is ascending)
-    const int cend = c0 + cnt;
-    while (bcur < bend) {
-      int idx = (bcur + lane < bend) ? blist[bcur + lane] : 0x7fffffff;
-      unsigned inb = __ballot_sync(0xffffffffu, idx < cend);
-      int m = __popc(inb);
-      for (int t = 0; t < m; t++) {
-        int j = __shfl_sync(0xffffffffu, idx, t) - c0;
-        const int *r = sm.rec[j];
-        int o = r[0];
-        // offset of this lane's cell in the footprint; outside -> the 0 weight
-        unsigned dx = min((unsigned)(lx - (int)(short)(o & 0xFFFF)), (unsigned)(2 * M + 1));
-        unsigned dy = min((unsigned)(ly - (o >> 16)), (unsigned)(2 * M + 1));
-        float w = __int_as_float(r[2 + dx]) * __int_as_float(r[2 + 2 * M + 2 + dy]);
+    locate(c0 + GS);
+    auto add = [&](int s, int2 b) {
+      const float wx = sm.wx[b.x + lx];
+      const float2 wy = sm.wy[(b.y + ly) >> 1];
+      const unsigned long long w0 = dup2(wx * wy.x), w1 = dup2(wx * wy.y);
+      const ulonglong2 *g = reinterpret_cast<const ulonglong2 *>(sm.g + s * GSTR);
 #pragma unroll
-        for (int zp = 0; zp < Z / 2; zp++) {
-          float4 v = sm.g[zp][j];
-          ar[2 * zp] = fmaf(w, v.x, ar[2 * zp]);
-          ai[2 * zp] = fmaf(w, v.y, ai[2 * zp]);
-          ar[2 * zp + 1] = fmaf(w, v.z, ar[2 * zp + 1]);
-          ai[2 * zp + 1] = fmaf(w, v.w, ai[2 * zp + 1]);
+      for (int q = 0; q < Z / 2; q++) {
+        const ulonglong2 t = g[q];
+        fma2(a0[2 * q], t.x, w0);
+        fma2(a1[2 * q], t.x, w1);
+        fma2(a0[2 * q + 1], t.y, w0);
+        fma2(a1[2 * q + 1], t.y, w1);
+      }
+    };
+    for (int k0 = 0; k0 < GS; k0 += 32) {
+      unsigned bits = __ballot_sync(0xffffffffu, (sm.mask[k0 + lane] >> wid) & 1);
+      while (bits) {
+        const int s0 = k0 + __ffs(bits) - 1;
+        bits &= bits - 1;
+        if constexpr (Z <= 4) {
+          // two samples in flight; the zero slot for a missing second
+          const int s1 = bits ? k0 + __ffs(bits) - 1 : GS;
+          bits &= bits - 1;
+          const int2 b0 = sm.base[s0];
+          const int2 b1 = s1 < GS ? sm.base[s1] : make_int2(GS * GXSLOT - xw, GS * GYSLOT - yw);
+          add(s0, b0);
+          add(s1, b1);
+        } else {
+          add(s0, sm.base[s0]);
         }
       }
-      bcur += m;
-      if (m < 32) break;
     }
-    __syncthreads();
   }
-  // store with coeff0 and the pre-FFT fftshift sign of the (2n+2m)^2 buffer
-  if (cx < twon && cy < twon) {
-    int sx = 1 - 2 * ((cx + M + 1) % 2), sy = 1 - 2 * ((cy + M + 1) % 2);
-    float sgn = (float)(sx * sy) * geo.coeff0;
+  const int cx = ix0 + lx, cy = iy0 + ly;
+  if (item.part >= 0) {
+    float2 *o = parts + (size_t)item.part * geo.nz * (TX * TY) + ly * TX + lx;
 #pragma unroll
     for (int z = 0; z < Z; z++)
-      if (z0 + z < geo.nz)
-        grid[((size_t)(z0 + z) * twon + cy) * twon + cx] = make_float2(ar[z] * sgn, ai[z] * sgn);
+      if (z0 + z < geo.nz) {
+        o[(size_t)(z0 + z) * (TX * TY)] = unpack2(a0[z]);
+        o[(size_t)(z0 + z) * (TX * TY) + TX] = unpack2(a1[z]);
+      }
+    return;
   }
+  // store with coeff0 and the pre-FFT fftshift sign of the (2n+2m)^2 buffer
+  // (2n is even: a lane's two rows are both inside the grid or both outside)
+  if (cx < twon && cy < twon) {
+    const int sx = 1 - 2 * ((cx + M + 1) % 2), sy = 1 - 2 * ((cy + M + 1) % 2);
+    const float sgn = (float)(sx * sy) * geo.coeff0;
+#pragma unroll
+    for (int z = 0; z < Z; z++)
+      if (z0 + z < geo.nz) {
+        float2 *o = grid + ((size_t)(z0 + z) * twon + cy) * twon + cx;
+        const float2 u = unpack2(a0[z]), w = unpack2(a1[z]);
+        o[0] = make_float2(u.x * sgn, u.y * sgn);
+        o[twon] = make_float2(-w.x * sgn, -w.y * sgn);
+      }
+  }
+}
+
+// The cells of split tiles: their partial sums added in the list's order.
+__global__ void __launch_bounds__(TX *TY)
+    grid_combine(float2 *__restrict__ grid, const float2 *__restrict__ parts,
+                 const GridSplit *__restrict__ splits, Geom geo) {
+  const GridSplit sp = splits[blockIdx.x];
+  const int z = blockIdx.y;
+  const int lx = threadIdx.x % TX, ly = threadIdx.x / TX;
+  const int cx = (sp.tile % geo.ntx) * TX + lx, cy = (sp.tile / geo.ntx) * TY + ly;
+  if (cx >= geo.twon || cy >= geo.twon) return;
+  float2 a = make_float2(0.f, 0.f);
+  for (int k = 0; k < sp.nparts; k++) {
+    const float2 b = parts[((size_t)(sp.part + k) * geo.nz + z) * (TX * TY) + threadIdx.x];
+    a.x += b.x;
+    a.y += b.y;
+  }
+  const int sx = 1 - 2 * ((cx + M + 1) % 2), sy = 1 - 2 * ((cy + M + 1) % 2);
+  const float sgn = (float)(sx * sy) * geo.coeff0;
+  grid[((size_t)z * geo.twon + cy) * geo.twon + cx] = make_float2(a.x * sgn, a.y * sgn);
 }
 
 // fftshift after the 2D FFT + divphi + circ (+ optional unpacking).
@@ -459,8 +493,8 @@ __global__ void __launch_bounds__(NTH, 2)
 // x 4 K-steps of tcgen05.mma (M = 128 cells, N = 64, K = 16) accumulating in
 // TMEM; while they run, the other CTA on the SM builds its chunk (one smem
 // stage per CTA, two CTAs per SM).  The epilogue undoes the scale and
-// stores like grid_blocks.  Weights and footprints are computed
-// exactly as grid_blocks computes them, once per geometry, into records laid
+// stores like grid_regs.  Weights and footprints are computed
+// exactly as grid_regs computes them, once per geometry, into records laid
 // out in the order of the tile lists (tile_records).
 constexpr int TCK = 64;                       // samples per chunk (one K block)
 constexpr int TCZ = 32;                       // slice pairs per tensor-gridding CTA
@@ -472,7 +506,7 @@ constexpr int TC_STAGE = TC_A + TC_B;
 constexpr int TC_THREADS = 512;
 
 // Per-(tile, sample) record, computed once per geometry with exactly the
-// arithmetic of grid_blocks, in the order of the tile lists:
+// arithmetic of grid_regs, in the order of the tile lists:
 // [0] tile-local footprint origin (lx0 | ly0 << 16), [1] index of the
 // sample's spectrum value p*n + (i + n/2) % n with the odd-i sign in bit 31,
 // [2..10] x-weights, [11..19] y-weights, [20..24] and [25..29] the byte
@@ -895,7 +929,7 @@ __global__ void __launch_bounds__(SW_THREADS)
       sample_pos(cs, rtab, p, i, (float)(2 * n), x0, y0, fx, fy);
       s_org[k] = (tile_origin(fx, X0, twon) & 0xFFFF) | (tile_origin(fy, Y0, twon) << 16);
       s_sg[k] = (i & 1) ? -SW_WSCALE : SW_WSCALE;
-      // the weights as the fp32 gridding computes them (grid_blocks)
+      // the weights as the fp32 gridding computes them (grid_regs)
 #pragma unroll
       for (int d = 0; d < 2 * M + 1; d++) {
         float w0 = etab[fx - M + d + n + M + EPAD] - x0;
@@ -920,7 +954,7 @@ __global__ void __launch_bounds__(SW_THREADS)
     if (o == 0x7FFF7FFF) continue;
     const int lx = (int)(short)(o & 0xFFFF) + dx, ly = (o >> 16) + dy;
     if (lx < 0 || lx >= SW_TX || ly < 0 || ly >= SW_TY) continue;
-    // the product as grid_blocks forms it, then the exact power-of-two scale and sign
+    // the product as grid_regs forms it, then the exact power-of-two scale and sign
     const float w = (s_w[k][0][dx] * s_w[k][1][dy]) * s_sg[k];
     const __half h = __float2half_rn(w);
     const uint32_t off = sw64_offset(ly * SW_TX + lx, k);
@@ -1682,8 +1716,10 @@ struct tcb_fourierrec {
   int *tile_order = nullptr;
   long long *toffs = nullptr;  // [ntiles+1] offsets into tlist
   int *tlist = nullptr;        // samples per tile (p*n+i)
-  long long *boffs = nullptr;  // [ntiles*16+1] offsets into blist
-  int *blist = nullptr;        // tile-local sample indices per 8x4 block
+  tcb::fr::GridItem *items = nullptr;   // work items of the fp32 gridding, longest first
+  tcb::fr::GridSplit *splits = nullptr; // tiles of several items
+  float2 *parts = nullptr;     // [slots][nz][TX*TY] partial sums of the split tiles
+  int nitems = 0, nsplits = 0;
   float2 *grid = nullptr;
   float2 *g32 = nullptr;  // fp32 staging of g (FLOAT16 only)
   cufftHandle plan1d = 0, plan2d = 0;
@@ -1698,7 +1734,7 @@ struct tcb_fourierrec {
   int own_cpc = 0;  // columns per block of the own column pass
   int t1_gw = tcb::fr::T1_GW;  // columns per group of the row-pass output (4, 8 or 16)
   bool own_rows_first = true;  // rows pass first (columns pass fused with deapodization)
-  int zblock = 0;  // pairs per gridding block (2/4/8/16; 0 = largest that fits nz)
+  int zblock = 0;  // most pairs per gridding CTA (2/4/8/16; 0 = the library's choice)
   int grid_mode = 0;          // TCB_GRID_FP32 or TCB_GRID_TENSOR
   bool out_f16 = false;       // fp16 output slices (set_output) with fp32 input
   bool spectrum_in = false;   // g already holds the projection FFT (set_input_spectrum)
@@ -1709,7 +1745,6 @@ struct tcb_fourierrec {
   float2 *tw = nullptr;  // per-stage twiddle table of the length-2n transforms
   float4 *dtab = nullptr;  // [n] deapodization terms (deapod_terms)
   int ntiles = 0;
-  size_t list_bytes = 0;
   // streamed-weight tensor-core gridding (16 x 16 tiles, chunks of 64 samples)
   int sw_nn = 0;                   // comps per CTA (64 or 128); 0 = not built
   int sw_ntx = 0, sw_ntiles = 0, sw_zgroups = 0;
@@ -1747,8 +1782,9 @@ void fr_release(tcb_fourierrec *h) {
   cudaFree(h->tile_order);
   cudaFree(h->toffs);
   cudaFree(h->tlist);
-  cudaFree(h->boffs);
-  cudaFree(h->blist);
+  cudaFree(h->items);
+  cudaFree(h->splits);
+  cudaFree(h->parts);
   cudaFree(h->grid);
   cudaFree(h->g32);
   cudaFree(h->t1);
@@ -1785,21 +1821,39 @@ void fr_release(tcb_fourierrec *h) {
   h->cs = nullptr;
   h->rtab = h->etab = nullptr;
   h->tile_order = nullptr;
-  h->toffs = h->boffs = nullptr;
-  h->tlist = h->blist = nullptr;
+  h->toffs = nullptr;
+  h->tlist = nullptr;
+  h->items = nullptr;
+  h->splits = nullptr;
+  h->parts = nullptr;
   h->grid = h->g32 = nullptr;
 }
 
 template <int Z>
 int launch_grid(tcb_fourierrec *h, const float2 *gc, cudaStream_t s) {
   const Geom &geo = h->geo;
-  unsigned zgroups = (unsigned)((h->nz + Z - 1) / Z);
-  grid_blocks<Z><<<(unsigned)h->ntiles * zgroups, NTH, sizeof(GridSmem<Z>), s>>>(
-      gc, h->grid, h->cs, h->rtab, h->etab, h->tile_order, h->toffs, h->tlist, h->boffs,
-      h->blist, geo);
+  const unsigned zgroups = (unsigned)((h->nz + Z - 1) / Z);
+  grid_regs<Z><<<(unsigned)h->nitems * zgroups, GT, sizeof(GridSmem<Z>), s>>>(
+      gc, h->grid, h->parts, h->cs, h->rtab, h->etab, h->items, h->toffs, h->tlist, geo);
   TCB_LAUNCH_CHECK();
   count_launch();
   return TCB_OK;
+}
+
+// Pairs per CTA of the fp32 gridding: the cheapest cover of nz.  A sample costs
+// a CTA about 28 issue slots for its weights and loop and 4.5 per pair; 16
+// pairs gain nothing over 8 (their registers leave two CTAs per SM, not three).
+int grid_pairs(size_t nz, int most) {
+  int best = 2;
+  double cost = 1e30;
+  for (int z = 2; z <= most; z *= 2) {
+    const double c = (double)((nz + z - 1) / z) * (28.0 + 4.5 * z);
+    if (c < cost) {
+      cost = c;
+      best = z;
+    }
+  }
+  return best;
 }
 
 int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
@@ -1911,12 +1965,18 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
   } else {
     StageTimer st("fr_gather", s);
     int rc;
-    const size_t zb = h->zblock ? (size_t)h->zblock : 16;
     h->grid_zero_fmt = h->own_n ? 1 : 0;  // every cell written, fp32
-    if (h->nz >= 16 && zb >= 16) rc = launch_grid<16>(h, gc, s);
-    else if (h->nz >= 8 && zb >= 8) rc = launch_grid<8>(h, gc, s);
-    else if (h->nz >= 4 && zb >= 4) rc = launch_grid<4>(h, gc, s);
-    else rc = launch_grid<2>(h, gc, s);
+    switch (grid_pairs(h->nz, h->zblock ? std::min(h->zblock, 8) : 8)) {
+      case 8: rc = launch_grid<8>(h, gc, s); break;
+      case 4: rc = launch_grid<4>(h, gc, s); break;
+      default: rc = launch_grid<2>(h, gc, s);
+    }
+    if (rc == TCB_OK && h->nsplits) {
+      grid_combine<<<dim3((unsigned)h->nsplits, (unsigned)h->nz), TX * TY, 0, s>>>(
+          h->grid, h->parts, h->splits, geo);
+      TCB_LAUNCH_CHECK();
+      count_launch();
+    }
     if (rc != TCB_OK) return rc;
   }
   const bool out_half = h->precision == TCB_FLOAT16 || h->out_f16;
@@ -1979,36 +2039,64 @@ int scan_counts(const int *d_counts, long long *d_offs, size_t count, long long 
   return TCB_OK;
 }
 
-// Build the per-tile and per-block sample lists (depends on theta and n only).
+// Build the per-tile sample lists (they depend on theta and n only) and the
+// work items of the fp32 gridding.
 int build_lists(tcb_fourierrec *h) {
   const Geom &geo = h->geo;
   const int nt = h->ntiles;
   int *counts = nullptr;
-  TCB_CUDA(cudaMalloc(&counts, (size_t)nt * NREG * sizeof(int)));
+  TCB_CUDA(cudaMalloc(&counts, (size_t)nt * sizeof(int)));
   int st = TCB_OK;
-  long long ntot = 0, nbtot = 0;
+  long long ntot = 0;
+  std::vector<int> cnt(nt);
+  // angles listed in steps near the golden section of nproj (and prime to it):
+  // the few lines of samples that grid_regs stages together then cross
+  // different warps' cells, so its warps reach the barrier together
+  int step = (int)(0.381966 * h->nproj) + 1;
+  while (std::gcd((size_t)step, h->nproj) != 1) step++;
   do {
-    list_tile_samples<TX, TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, 0, counts, nullptr,
+    list_tile_samples<TX, TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, step, 0, counts, nullptr,
                                                 nullptr);
     if (cudaGetLastError() != cudaSuccess) { st = TCB_ERR_CUDA; break; }
     if ((st = scan_counts(counts, h->toffs, nt, ntot)) != TCB_OK) break;
-    if (cudaMalloc(&h->tlist, std::max<long long>(ntot, 1) * sizeof(int)) != cudaSuccess) {
+    if (cudaMemcpy(cnt.data(), counts, (size_t)nt * sizeof(int), cudaMemcpyDeviceToHost) !=
+        cudaSuccess) {
+      st = TCB_ERR_CUDA;
+      break;
+    }
+    // items, longest first (then in tile order)
+    const long long len = std::max<long long>(1024, ntot / (8 * 148) / GS * GS);
+    std::vector<GridItem> items;
+    std::vector<GridSplit> splits;
+    int slots = 0;
+    for (int t = 0; t < nt; t++) {
+      const int np = (int)((cnt[t] + len - 1) / len);
+      if (np > 1) splits.push_back({t, slots, np});
+      for (int k = 0; k < std::max(np, 1); k++)
+        items.push_back({t, (int)(k * len), (int)std::min<long long>(len, cnt[t] - k * len),
+                         np > 1 ? slots + k : -1});
+      if (np > 1) slots += np;
+    }
+    std::stable_sort(items.begin(), items.end(),
+                     [](const GridItem &a, const GridItem &b) { return a.count > b.count; });
+    h->nitems = (int)items.size();
+    h->nsplits = (int)splits.size();
+    if (cudaMalloc(&h->tlist, std::max<long long>(ntot, 1) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&h->items, items.size() * sizeof(GridItem)) != cudaSuccess ||
+        (slots && (cudaMalloc(&h->splits, splits.size() * sizeof(GridSplit)) != cudaSuccess ||
+                   cudaMalloc(&h->parts, (size_t)slots * h->nz * TX * TY * sizeof(float2)) !=
+                       cudaSuccess))) {
       st = TCB_ERR_OUT_OF_MEMORY;
       break;
     }
-    list_tile_samples<TX, TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, 1, nullptr, h->toffs,
+    cudaError_t e = cudaMemcpy(h->items, items.data(), items.size() * sizeof(GridItem),
+                               cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && slots)
+      e = cudaMemcpy(h->splits, splits.data(), splits.size() * sizeof(GridSplit),
+                     cudaMemcpyHostToDevice);
+    list_tile_samples<TX, TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, step, 1, nullptr, h->toffs,
                                                 h->tlist);
-    list_block_samples<<<nt, NTH>>>(h->cs, h->rtab, geo, h->toffs, h->tlist, 0, counts,
-                                    nullptr, nullptr);
-    if (cudaGetLastError() != cudaSuccess) { st = TCB_ERR_CUDA; break; }
-    if ((st = scan_counts(counts, h->boffs, (size_t)nt * NREG, nbtot)) != TCB_OK) break;
-    if (cudaMalloc(&h->blist, std::max<long long>(nbtot, 1) * sizeof(int)) != cudaSuccess) {
-      st = TCB_ERR_OUT_OF_MEMORY;
-      break;
-    }
-    list_block_samples<<<nt, NTH>>>(h->cs, h->rtab, geo, h->toffs, h->tlist, 1, nullptr,
-                                    h->boffs, h->blist);
-    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
       set_error("fourierrec: list construction failed: %s", cudaGetErrorString(e));
       st = TCB_ERR_CUDA;
@@ -2016,9 +2104,11 @@ int build_lists(tcb_fourierrec *h) {
     }
   } while (0);
   cudaFree(counts);
-  if (st == TCB_ERR_OUT_OF_MEMORY) set_error("fourierrec: out of memory for sample lists");
+  if (st == TCB_ERR_OUT_OF_MEMORY) {
+    cudaGetLastError();
+    set_error("fourierrec: out of memory for sample lists");
+  }
   if (st == TCB_ERR_CUDA && tcb_last_error()[0] == 0) set_error("fourierrec: list kernel failed");
-  h->list_bytes = (size_t)(ntot + nbtot) * sizeof(int);
   return st;
 }
 
@@ -2045,7 +2135,7 @@ int sw_build(tcb_fourierrec *h, bool with_lo) {
     if (cudaMalloc(&counts, (size_t)nt * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&h->sw_toffs, ((size_t)nt + 1) * sizeof(long long)) != cudaSuccess)
       return oom("tile offsets");
-    list_tile_samples<SW_TX, SW_TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, 0, counts, nullptr,
+    list_tile_samples<SW_TX, SW_TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, 1, 0, counts, nullptr,
                                                       nullptr);
     TCB_CUDA(cudaGetLastError());
     long long total = 0;
@@ -2055,7 +2145,7 @@ int sw_build(tcb_fourierrec *h, bool with_lo) {
     if (st != TCB_OK) return st;
     if (cudaMalloc(&h->sw_tlist, std::max<long long>(total, 1) * sizeof(int)) != cudaSuccess)
       return oom("tile lists");
-    list_tile_samples<SW_TX, SW_TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, 1, nullptr,
+    list_tile_samples<SW_TX, SW_TY><<<nt, SETUP_NT>>>(h->cs, h->rtab, geo, 1, 1, nullptr,
                                                       h->sw_toffs, h->sw_tlist);
     TCB_CUDA(cudaGetLastError());
   }
@@ -2206,7 +2296,6 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
   FR_ALLOC(h->etab, (2 * n + 2 * M + 1 + 2 * EPAD) * sizeof(float));
   FR_ALLOC(h->tile_order, h->ntiles * sizeof(int));
   FR_ALLOC(h->toffs, (h->ntiles + 1) * sizeof(long long));
-  FR_ALLOC(h->boffs, ((size_t)h->ntiles * NREG + 1) * sizeof(long long));
   FR_ALLOC(h->grid, nz * 4 * n * n * sizeof(float2));
   FR_ALLOC(h->dtab, n * sizeof(float4));
   if (precision == TCB_FLOAT16) FR_ALLOC(h->g32, nz * nproj * n * sizeof(float2));
@@ -2241,11 +2330,14 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
   }
   int st = build_lists(h);
   if (st != TCB_OK) return fail(st);
-  e = cudaFuncSetAttribute(grid_blocks<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(GridSmem<16>));
+  e = cudaFuncSetAttribute(grid_regs<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GridSmem<8>));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(grid_blocks<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(GridSmem<8>));
+    e = cudaFuncSetAttribute(grid_regs<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(GridSmem<4>));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(grid_regs<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(GridSmem<2>));
   if (e != cudaSuccess) {
     set_error("tcb_fourierrec_create: smem attribute failed: %s", cudaGetErrorString(e));
     return fail(TCB_ERR_CUDA);
