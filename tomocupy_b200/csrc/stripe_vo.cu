@@ -206,23 +206,72 @@ __global__ void __launch_bounds__(VO_MED_T)
 
 // _rs_dead3's column variation: diff[z][x] = sum_p |tomo - uniform_filter1d(
 // tomo, 10, axis=0)| (reflect mode; window p-5 .. p+4, a float64 running sum
-// divided by 10 and rounded, as scipy's filter), accumulated in float32 in
-// angle order.  One thread per column.
-__global__ void vo_dead_diff(const float *__restrict__ tomo, size_t pstride, size_t zstride,
-                             int nproj, int nz, int ni, float *__restrict__ diff) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.y;
-  if (x >= ni) return;
-  const float *col = tomo + (size_t)z * zstride + x;
-  auto v = [&](int p) { return (double)col[(size_t)reflect_idx(p, nproj) * pstride]; };
-  double run = 0.0;
-  for (int p = -5; p <= 4; p++) run += v(p);
+// divided by 10 and rounded, as scipy's filter).  A thread takes one of the
+// DD_SEG runs of angles of a column, with its own running sum; the runs' float32
+// sums are added in angle order.  One thread per column had 128 CTAs of serial
+// chains on the chip (0.6 ms at 720 angles x 16 rows x 1024 columns); the chain
+// bounds it, not the one read of the data, so it is cut into 16
+// (with the medians below: 1.13 -> 0.13 ms).
+constexpr int DD_SEG = 16;
+__global__ void __launch_bounds__(32 * DD_SEG)
+    vo_dead_diff(const float *__restrict__ tomo, size_t pstride, size_t zstride, int nproj,
+                 int nz, int ni, float *__restrict__ diff) {
+  __shared__ float part[DD_SEG][32];
+  const int lane = threadIdx.x, seg = threadIdx.y;
+  const int x = blockIdx.x * 32 + lane, z = blockIdx.y;
+  const int len = (nproj + DD_SEG - 1) / DD_SEG;
+  const int p0 = seg * len, p1 = min(nproj, p0 + len);
   float acc = 0.f;
-  for (int p = 0; p < nproj; p++) {
-    const float m = (float)(run / 10.0);
-    acc += fabsf(col[(size_t)p * pstride] - m);
-    run += v(p + 5) - v(p - 5);
+  if (x < ni && p0 < p1) {
+    const float *col = tomo + (size_t)z * zstride + x;
+    auto v = [&](int p) {  // reflected: nproj >= 12, one fold suffices
+      const int q = p < 0 ? -1 - p : p >= nproj ? 2 * nproj - 1 - p : p;
+      return (double)col[(size_t)q * pstride];
+    };
+    double run = 0.0;
+    for (int p = p0 - 5; p <= p0 + 4; p++) run += v(p);
+    for (int p = p0; p < p1; p++) {
+      const float m = (float)(run / 10.0);
+      acc += fabsf(col[(size_t)p * pstride] - m);
+      run += v(p + 5) - v(p - 5);
+    }
   }
-  diff[(size_t)z * ni + x] = acc;
+  part[seg][lane] = acc;
+  __syncthreads();
+  if (seg == 0 && x < ni) {
+    for (int k = 1; k < DD_SEG; k++) acc += part[k][lane];
+    diff[(size_t)z * ni + x] = acc;
+  }
+}
+
+// Median over w (odd) columns, reflect mode, of the row statistics in[z][x]:
+// each thread finds the value of rank w/2 of its window by counting.  There are
+// too few rows of statistics to fill the chip with sliding windows (vo_median_x
+// took 0.5 ms for 16 rows of 1024), and w^2 comparisons cost a thread 4000 loads.
+__global__ void __launch_bounds__(256)
+    vo_median_row(const float *__restrict__ in, float *__restrict__ out, int ni, int w) {
+  extern __shared__ float win[];  // [256 + w - 1] values of the block's windows
+  const int x0 = blockIdx.x * 256, z = blockIdx.y, h = w / 2;
+  for (int k = threadIdx.x; k < 256 + w - 1; k += 256)
+    win[k] = in[(size_t)z * ni + reflect_idx(x0 - h + k, ni)];
+  __syncthreads();
+  const int x = x0 + threadIdx.x;
+  if (x >= ni) return;
+  const float *v = win + threadIdx.x;
+  float med = v[h];
+  for (int j = 0; j < w; j++) {
+    const float c = v[j];
+    int lt = 0, le = 0;
+    for (int k = 0; k < w; k++) {
+      lt += v[k] < c;
+      le += v[k] <= c;
+    }
+    if (lt <= h && le > h) {
+      med = c;
+      break;
+    }
+  }
+  out[(size_t)z * ni + x] = med;
 }
 
 // Mean over ranks [nd, nproj - nd) of sorted and smoothed columns -> l1, l2.
@@ -519,7 +568,7 @@ extern "C" int tcb_stripe_vo_apply(tcb_stripe_vo *h, float *tomo, size_t pstride
   const int np = (int)h->nproj, nz = (int)h->nz, ni = (int)h->ni;
   // at least a full warp of threads (the shuffle stages)
   const int p2 = std::max(pow2_at_least(np), 128), n2 = pow2_at_least(ni);
-  const dim3 cgrid(ceil_div(h->ni, 128), nz), pgrid(ceil_div(h->ni, 128), nz, 16);
+  const dim3 pgrid(ceil_div(h->ni, 128), nz, 16);
   const int nd = (int)(0.5 * 0.1 * np);  // drop_ratio 0.1
   const int dsm = (int)(2 * h->ni * 4 + n2 * 4);
   // sorts read the column-contiguous copy tt
@@ -543,8 +592,10 @@ extern "C" int tcb_stripe_vo_apply(tcb_stripe_vo *h, float *tomo, size_t pstride
   // 1. dead stripes
   {
     StageTimer st("stripe_vo_dead", s);
-    vo_dead_diff<<<cgrid, 128, 0, s>>>(tomo, pstride, zstride, np, nz, ni, h->l1);
-    median(h->l1, h->l2, 1, h->la);
+    vo_dead_diff<<<dim3(ceil_div(h->ni, 32), nz), dim3(32, DD_SEG), 0, s>>>(
+        tomo, pstride, zstride, np, nz, ni, h->l1);
+    vo_median_row<<<dim3(ceil_div(h->ni, 256), nz), 256, (256 + h->la - 1) * sizeof(float), s>>>(
+        h->l1, h->l2, ni, h->la);
     vo_detect<<<nz, 256, dsm, s>>>(h->l1, h->l2, ni, n2, h->snr, 1, h->fact, h->mask, h->nbr);
     vo_dead_interp<<<pgrid, 128, 0, s>>>(tomo, pstride, zstride, np, ni, h->mask, h->nbr);
     TCB_LAUNCH_CHECK();
