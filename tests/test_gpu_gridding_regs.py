@@ -30,6 +30,11 @@ def test_register_gridding_vs_float64(cuda, n, nproj, nz):
     theta = (np.arange(nproj) * np.pi / nproj + 0.01).astype(np.float32)
     want = np_tomo.fourierrec_pairs(g, theta, n, np.float64)
     th = torch.as_tensor(theta, device=cuda)
+    # pixels on the circle itself (4x^2 + 4y^2 = 1): float32 and float64 may
+    # decide differently
+    c = (2 * np.arange(n) - n) / n
+    inside = np.abs(c[:, None] ** 2 + c[None, :] ** 2 - 1) > 1e-5
+    want = np.ascontiguousarray(want * inside)
     out = []
     for pairs in (0, 2, 4):
         op = cfunc_fourierrec(nproj, nz, n, th)
@@ -39,6 +44,6 @@ def test_register_gridding_vs_float64(cuda, n, nproj, nz):
         f = torch.full((nz, n, n, 2), float("nan"), device=cuda)
         op.backprojection(f, gd, torch.cuda.current_stream())
         out.append(f.cpu().numpy())
-        assert rel_l2(out[-1], want.view(np.float64).reshape(nz, n, n, 2)) < 5e-5
+        assert rel_l2(out[-1] * inside[None, :, :, None], want.view(np.float64).reshape(nz, n, n, 2)) < 5e-5
     # the pairs of a CTA do not change the order of a cell's sum
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
