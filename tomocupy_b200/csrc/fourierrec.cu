@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft_mixed.cuh"
 #include "fft_pow2.cuh"
 #include "tcgen05.cuh"
 
@@ -1454,6 +1455,50 @@ __global__ void deapod_kernel(const float2 *__restrict__ grid, OutT *__restrict_
             tx, ty, tz, geo, unpack);
 }
 
+// cuFFT's pruned inverse transform (2n not a power of two, or cuFFT forced): the
+// n kept columns of the row-transformed grid, transposed to t[z][c][y], so that
+// the column transforms run on contiguous lines (8 pairs at 2n = 4896: 2.2 ms
+// strided within the grid, 0.75 ms contiguous and 0.36 ms for this copy).
+// 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256)
+    crop_transpose(const float2 *__restrict__ grid, float2 *__restrict__ t, int n) {
+  __shared__ float2 tile[32][33];
+  const int twon = 2 * n, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+  const float2 *src = grid + (size_t)blockIdx.z * twon * twon + n / 2;
+  float2 *dst = t + (size_t)blockIdx.z * n * twon;
+  for (int k = w; k < 32; k += 8)
+    if (y0 + k < twon && c0 + lane < n)
+      tile[k][lane] = src[(size_t)(y0 + k) * twon + c0 + lane];
+  __syncthreads();
+  for (int k = w; k < 32; k += 8)
+    if (c0 + k < n && y0 + lane < twon) dst[(size_t)(c0 + k) * twon + y0 + lane] = tile[lane][k];
+}
+
+// deapod_kernel on the transposed columns t[z][c][y].
+template <typename OutT>
+__global__ void __launch_bounds__(256)
+    deapod_transposed(const float2 *__restrict__ t, OutT *__restrict__ f,
+                      const float4 *__restrict__ dtab, Geom geo, int unpack) {
+  __shared__ float2 tile[32][33];
+  const int n = geo.n, twon = geo.twon, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, z = blockIdx.z;
+  const float2 *src = t + (size_t)z * n * twon + n / 2 + 1;
+  for (int k = w; k < 32; k += 8)
+    if (x0 + k < n && y0 + lane < n) tile[k][lane] = src[(size_t)(x0 + k) * twon + y0 + lane];
+  __syncthreads();
+  const int tx = x0 + lane;
+  if (tx >= n) return;
+  for (int k = w; k < 32; k += 8) {
+    const int ty = y0 + k;
+    if (ty < n)
+      store_out(f,
+                deapod_terms_value(tile[lane][k], __ldg(dtab + tx), __ldg(dtab + ty),
+                                   geo.mu * (n * n), geo.nproj, (float)(1 - n % 4)),
+                tx, ty, z, geo, unpack);
+  }
+}
+
 // Own pruned inverse 2D FFT for power-of-two 2n (N = 2n).
 // Pass 1 (columns): CPC adjacent columns x of one pair's N x N grid per
 // block; the inverse FFT along y keeps rows y' in [n/2 + 1, 3n/2 + 1), the
@@ -1728,6 +1773,9 @@ struct tcb_fourierrec {
   // transforms over only the n columns [n/2, 3n/2) that deapodization reads.
   cufftHandle plan_rows = 0, plan_cols = 0;
   bool pruned = false;
+  // the same two passes on the library's mixed-radix lines (mix.n = 2n, else 0)
+  tcb::mixfft::Plan mix;
+  float2 *mixtw = nullptr;
   // Own pruned FFT (rows pass, then columns pass fused with deapodization,
   // or the reverse) when 2n is a power of two in [256, 8192]: own_n = 2n,
   // else 0.
@@ -1742,7 +1790,9 @@ struct tcb_fourierrec {
   unsigned *amax = nullptr;   // max |G| bits for the tensor-core gridding scale
   int *trec = nullptr;        // per-(tile, sample) records (tensor-core gridding)
   int *tc_err = nullptr;      // set by a tensor-core gridding wait that timed out
-  float2 *t1 = nullptr;  // first-pass output: [nz][2n][n] rows first, [nz][n][2n] columns first
+  // first-pass output: [nz][2n][n] own rows first, [nz][n][2n] own columns first
+  // and cuFFT's transposed kept columns
+  float2 *t1 = nullptr;
   float2 *tw = nullptr;  // per-stage twiddle table of the length-2n transforms
   float4 *dtab = nullptr;  // [n] deapodization terms (deapod_terms)
   int ntiles = 0;
@@ -1789,6 +1839,8 @@ void fr_release(tcb_fourierrec *h) {
   cudaFree(h->grid);
   cudaFree(h->g32);
   cudaFree(h->t1);
+  cudaFree(h->mixtw);
+  h->mixtw = nullptr;
   cudaFree(h->tw);
   cudaFree(h->dtab);
   h->dtab = nullptr;
@@ -1872,7 +1924,7 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
     gc = h->g32;
   }
   TCB_CUFFT(cufftSetStream(h->plan1d, s));
-  if (h->own_n) {
+  if (h->own_n || h->mix.n) {
   } else if (h->pruned) {
     TCB_CUFFT(cufftSetStream(h->plan_rows, s));
     TCB_CUFFT(cufftSetStream(h->plan_cols, s));
@@ -2000,14 +2052,34 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
   }
   {
     StageTimer st("fr_fft2d", s);
-    if (h->pruned) {
+    if (h->mix.n) {
+      const size_t sm = mixfft::smem_bytes(h->mix.n);
+      const int lo = geo.n / 2, nt = h->mix.threads;
+      mixfft::ifft_lines<<<(unsigned)(2 * h->n * h->nz), nt, sm, s>>>(h->grid, h->mixtw, h->mix,
+                                                                      lo, lo + geo.n);
+      crop_transpose<<<dim3(ceil_div(h->n, 32), ceil_div(2 * h->n, 32), (unsigned)h->nz), 256, 0,
+                       s>>>(h->grid, h->t1, geo.n);
+      mixfft::ifft_lines<<<(unsigned)(h->n * h->nz), nt, sm, s>>>(h->t1, h->mixtw, h->mix, lo + 1,
+                                                                  lo + 1 + geo.n);
+      TCB_LAUNCH_CHECK();
+      count_launch(3);
+    } else if (h->pruned) {
       // separable: all rows along x, then the kept columns along y, per pair
       TCB_CUFFT(cufftExecC2C(h->plan_rows, (cufftComplex *)h->grid, (cufftComplex *)h->grid,
                              CUFFT_INVERSE));
-      const size_t plane = (size_t)geo.twon * geo.twon;
-      for (size_t z = 0; z < h->nz; z++) {
-        cufftComplex *c = (cufftComplex *)(h->grid + z * plane + h->n / 2);
-        TCB_CUFFT(cufftExecC2C(h->plan_cols, c, c, CUFFT_INVERSE));
+      if (h->t1) {
+        crop_transpose<<<dim3(ceil_div(h->n, 32), ceil_div(2 * h->n, 32), (unsigned)h->nz), 256,
+                         0, s>>>(h->grid, h->t1, geo.n);
+        TCB_LAUNCH_CHECK();
+        count_launch();
+        TCB_CUFFT(cufftExecC2C(h->plan_cols, (cufftComplex *)h->t1, (cufftComplex *)h->t1,
+                               CUFFT_INVERSE));
+      } else {
+        const size_t plane = (size_t)geo.twon * geo.twon;
+        for (size_t z = 0; z < h->nz; z++) {
+          cufftComplex *c = (cufftComplex *)(h->grid + z * plane + h->n / 2);
+          TCB_CUFFT(cufftExecC2C(h->plan_cols, c, c, CUFFT_INVERSE));
+        }
       }
     } else {
       TCB_CUFFT(cufftExecC2C(h->plan2d, (cufftComplex *)h->grid, (cufftComplex *)h->grid,
@@ -2016,11 +2088,19 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
   }
   {
     StageTimer st("fr_deapod", s);
-    dim3 blk(32, 8), grd(ceil_div(h->n, 32), ceil_div(h->n, 8), (unsigned)h->nz);
-    if (out_half)
-      deapod_kernel<__half><<<grd, blk, 0, s>>>(h->grid, (__half *)f, h->dtab, geo, unpack);
-    else
-      deapod_kernel<float><<<grd, blk, 0, s>>>(h->grid, (float *)f, h->dtab, geo, unpack);
+    if (h->pruned && h->t1) {
+      const dim3 grd(ceil_div(h->n, 32), ceil_div(h->n, 32), (unsigned)h->nz);
+      if (out_half)
+        deapod_transposed<__half><<<grd, 256, 0, s>>>(h->t1, (__half *)f, h->dtab, geo, unpack);
+      else
+        deapod_transposed<float><<<grd, 256, 0, s>>>(h->t1, (float *)f, h->dtab, geo, unpack);
+    } else {
+      dim3 blk(32, 8), grd(ceil_div(h->n, 32), ceil_div(h->n, 8), (unsigned)h->nz);
+      if (out_half)
+        deapod_kernel<__half><<<grd, blk, 0, s>>>(h->grid, (__half *)f, h->dtab, geo, unpack);
+      else
+        deapod_kernel<float><<<grd, blk, 0, s>>>(h->grid, (float *)f, h->dtab, geo, unpack);
+    }
     TCB_LAUNCH_CHECK();
     count_launch();
   }
@@ -2429,12 +2509,47 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
   }
   if (r == CUFFT_SUCCESS && !h->pruned)
     r = cufftPlanMany(&h->plan2d, 2, len2, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, (int)nz);
-  if (r == CUFFT_SUCCESS && h->pruned && !h->own_n) {
+  if (h->pruned && !h->own_n) {
+    // the columns on a transposed copy; within the grid when the copy does not fit
+    if (cudaMalloc(&h->t1, nz * n * N2 * sizeof(float2)) != cudaSuccess) {
+      cudaGetLastError();
+      h->t1 = nullptr;
+    }
+    // 2n a product of primes up to 17 (8 pairs at 4896 =
+    // 17 18 16: 1.73 ms with the copy between the passes; cuFFT's passes 4.9)
+    std::vector<float2> twh;
+    if (h->t1 && own_sel && N2 <= (size_t)mixfft::MAX_N) h->mix = mixfft::make_plan((int)N2, twh);
+    if (h->mix.n) {
+      if (cudaMalloc(&h->mixtw, twh.size() * sizeof(float2)) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("tcb_fourierrec_create: out of device memory for the FFT tables");
+        return fail(TCB_ERR_OUT_OF_MEMORY);
+      }
+      e = cudaMemcpy(h->mixtw, twh.data(), twh.size() * sizeof(float2), cudaMemcpyHostToDevice);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mixfft::ifft_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)mixfft::smem_bytes(mixfft::MAX_N));
+      if (e != cudaSuccess) {
+        set_error("tcb_fourierrec_create: FFT setup failed: %s", cudaGetErrorString(e));
+        return fail(TCB_ERR_CUDA);
+      }
+    }
+  }
+  if (r == CUFFT_SUCCESS && h->pruned && !h->own_n && !h->mix.n) {
     int lr[1] = {(int)(2 * n)};
     r = cufftPlanMany(&h->plan_rows, 1, lr, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
                       (int)(2 * n * nz));
+    if (r == CUFFT_SUCCESS && h->t1 &&
+        cufftPlanMany(&h->plan_cols, 1, lr, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
+                      (int)(n * nz)) != CUFFT_SUCCESS) {
+      // no room for this plan's workspace beside the copy
+      cudaGetLastError();
+      cudaFree(h->t1);
+      h->t1 = nullptr;
+      h->plan_cols = 0;
+    }
     int emb[1] = {(int)(2 * n)};
-    if (r == CUFFT_SUCCESS)
+    if (r == CUFFT_SUCCESS && !h->t1)
       r = cufftPlanMany(&h->plan_cols, 1, lr, emb, (int)(2 * n), 1, emb, (int)(2 * n), 1,
                         CUFFT_C2C, (int)n);
   }
