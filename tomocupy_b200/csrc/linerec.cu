@@ -386,15 +386,18 @@ __global__ void __launch_bounds__(BX *BY)
 // which is what the bilinear sum of lr_interp rounds to when its other two
 // weights are zero; the sums are bit-identical to backproject_full_tma's.  The
 // other row's two samples enter there times zero, which matters only when they
-// are not finite: `bad` gathers 0 * p of every row and is added at the end.
+// are not finite: the sum of that row (the neighbouring slice's) is added times
+// zero at the end.
 //
 // Z consecutive slices per thread (8, or 4 where that leaves fewer slices
-// unused) share the column arithmetic; slices go in pairs through packed
-// FP32 instructions.  The two 4-byte shared-memory loads per row and angle
-// bound it: 2 (Z + 2) / Z per update, 3600 updates/ns over the chip at Z = 8
-// against 16 loads and 45 instructions per update of the bilinear form.
-// 1024^2 x 16 slices x 720 angles: 6.1 ms, against 15.2 ms for the bilinear form.
+// unused) share the column arithmetic; rows go in pairs through packed FP32
+// instructions.  Bound: instruction issue, about 20 for the column, 2 (Z + 2)
+// loads and 1.5 (Z + 2) packed operations per angle; the loads alone would allow
+// 3600 updates/ns over the chip at Z = 8.
+// 1024^2 x 16 slices x 720 angles: 4.9 ms, against 15.2 ms for the bilinear form.
 constexpr int RAC = 16;  // angles per stage
+constexpr float FLOOR_MAGIC = 8388608.f;  // 2^23
+constexpr int FLOOR_BITS = 0x4B000000;    // its bits
 
 template <int Z> struct RowBox {
   static constexpr int VR = Z + 2;
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(BX *BY)
   using B = RowBox<Z>;
   extern __shared__ uint8_t lr_raw[];
   uint8_t *sm = lr_raw + ((128u - (smem_u32(lr_raw) & 127u)) & 127u);
-  __shared__ float4 s_t[2][RAC];  // cos, sin, box origin (integer bits)
+  __shared__ float4 s_t[2][RAC];  // cos, sin, box origin plus FLOOR_BITS, box origin (integer bits)
   __shared__ uint64_t bar[2];
   const int tx = blockIdx.x * BX + threadIdx.x;
   const int ty = blockIdx.y * BY + threadIdx.y;
@@ -444,6 +447,7 @@ __global__ void __launch_bounds__(BX *BY)
   const int v0 = tz0 + sz - 1;  // box row r is sinogram row v0 + r; slice s reads row s + 1
   const int nch = (nproj + RAC - 1) / RAC;
   const float fx = (float)(tx - n / 2), fy = (float)(ty - n / 2), fh = (float)(n / 2);
+  const float last = (float)(n - 1);
   // slices whose fraction of v is 0 (slice 0; beyond 256 rows most, where
   // v - 1e-5 rounds to v): their bilinear sum adds the two samples the other way round
   int flip = 0;
@@ -452,9 +456,9 @@ __global__ void __launch_bounds__(BX *BY)
     if (v == (float)(int)(v - 1e-5f)) flip |= 1 << k;
   }
   // rows 1 .. Z in pairs, and the outer rows 0, Z + 1 as one pair
-  unsigned long long acc[Z / 2], bad[Z / 2], edge = 0ull;
+  unsigned long long acc[Z / 2], edge = 0ull;
 #pragma unroll
-  for (int k = 0; k < Z / 2; k++) acc[k] = bad[k] = 0ull;
+  for (int k = 0; k < Z / 2; k++) acc[k] = 0ull;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -469,8 +473,10 @@ __global__ void __launch_bounds__(BX *BY)
                                fminf(ct * x0 + stt * (y0 + BY - 1),
                                      ct * (x0 + BX - 1) + stt * (y0 + BY - 1))) +
                          n / 2;
-      const int u0 = ((int)floorf(umin) - 1) & ~3;  // down to a multiple of 4
-      s_t[st][tid] = make_float4(ct, stt, __int_as_float(u0), 0.f);
+      // down to a multiple of 4; the tile's u span at most sqrt(31^2 + 7^2) < 32,
+      // so their samples are 1 .. 37 from here
+      const int u0 = ((int)floorf(umin) - 1) & ~3;
+      s_t[st][tid] = make_float4(ct, stt, __int_as_float(u0 + FLOOR_BITS), __int_as_float(u0));
     }
   };
   auto issue = [&](int cc, int st) {  // one thread
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(BX *BY)
     mbar_expect_tx(&bar[st], (uint32_t)(cnt * TUW * B::VR * 4));
     for (int a = 0; a < cnt; a++)
       tma_load_3d(sm + st * B::STAGE + a * B::BYTES, &map, &bar[st],
-                  __float_as_int(s_t[st][a].z), t0 + a, v0);
+                  __float_as_int(s_t[st][a].w), t0 + a, v0);
   };
   prep(0, 0);
   __syncthreads();
@@ -498,30 +504,24 @@ __global__ void __launch_bounds__(BX *BY)
       for (int k = 0; k < cnt; k++) {
         const float4 t = s_t[st][k];
         float u = lr_u(t.x, t.y, fx, fy, fh);
-        const int ur = (int)(u - 1e-5f);
-        if (!((ur >= 0) & (ur < n - 1))) continue;
-        u = u - ur;
-        const int bu = ur - __float_as_int(t.z);
+        // ur = (int)(u - 1e-5f) without the conversion units: adding 2^23 rounded
+        // down leaves floor in the low bits (u - 1e-5 in (-1, 0) truncates to 0)
+        const float tr = u - 1e-5f;
+        const float fl = __fadd_rd(fmaxf(tr, 0.f), FLOOR_MAGIC);
+        const float uf = fl - FLOOR_MAGIC;
+        if (tr <= -1.f || uf >= last) continue;  // ur < 0 or ur >= n - 1
+        u = u - uf;
+        // the box holds every ur + 1 of the tile (see prep); clamped all the same
+        const int bu = min(max(__float_as_int(fl) - __float_as_int(t.z), 0), TUW - 2);
+        const float *bx = reinterpret_cast<const float *>(sm + st * B::STAGE + k * B::BYTES) + bu;
         float d0[B::VR], d1[B::VR];
-        if ((bu >= 0) & (bu < TUW - 1)) {
-          const float *bx = reinterpret_cast<const float *>(sm + st * B::STAGE + k * B::BYTES) + bu;
 #pragma unroll
-          for (int r = 0; r < B::VR; r++) {
-            d0[r] = bx[r * TUW];
-            d1[r] = bx[r * TUW + 1];
-          }
-        } else {
-          const float *g = data + ur + (size_t)(t0 + k) * n;
-#pragma unroll
-          for (int r = 0; r < B::VR; r++) {
-            const int v = v0 + r;
-            const bool in = v >= 0 && v < nz;
-            d0[r] = in ? g[(size_t)v * n * nproj] : 0.f;
-            d1[r] = in ? g[(size_t)v * n * nproj + 1] : 0.f;
-          }
+        for (int r = 0; r < B::VR; r++) {
+          d0[r] = bx[r * TUW];
+          d1[r] = bx[r * TUW + 1];
         }
         const float w = 1 - u;
-        const unsigned long long uu = lr_pack(u, u), ww = lr_pack(w, w), z2 = 0ull;
+        const unsigned long long uu = lr_pack(u, u), ww = lr_pack(w, w);
         auto one = [&](int r, int s) {  // row r of slice s
           return (flip >> s) & 1 ? __fmaf_rn(d0[r], w, __fmul_rn(d1[r], u))
                                  : __fmaf_rn(d1[r], u, __fmul_rn(d0[r], w));
@@ -533,11 +533,10 @@ __global__ void __launch_bounds__(BX *BY)
               flipped ? lr_pack(one(r, 2 * q), one(r + 1, 2 * q + 1))
                       : lr_lerp2(lr_pack(d0[r], d0[r + 1]), lr_pack(d1[r], d1[r + 1]), uu, ww);
           asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[q]) : "l"(p));
-          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(bad[q]) : "l"(p), "l"(z2));
         }
         const unsigned long long p =
             lr_lerp2(lr_pack(d0[0], d0[Z + 1]), lr_pack(d1[0], d1[Z + 1]), uu, ww);
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(edge) : "l"(p), "l"(z2));
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(edge) : "l"(p));
       }
     };
     if (active) {
@@ -559,18 +558,15 @@ __global__ void __launch_bounds__(BX *BY)
     return;
   }
   if (!active) return;
-  float a[Z], b[Z + 2];
+  float a[Z + 2];
 #pragma unroll
   for (int q = 0; q < Z / 2; q++) {
-    const float2 va = lr_unpack(acc[q]), vb = lr_unpack(bad[q]);
-    a[2 * q] = va.x;
-    a[2 * q + 1] = va.y;
-    b[2 * q + 1] = vb.x;
-    b[2 * q + 2] = vb.y;
+    const float2 v = lr_unpack(acc[q]);
+    a[2 * q + 1] = v.x;
+    a[2 * q + 2] = v.y;
   }
-  const float2 ve = lr_unpack(edge);
-  b[0] = ve.x;
-  b[Z + 1] = ve.y;
+  a[0] = lr_unpack(edge).x;
+  a[Z + 1] = lr_unpack(edge).y;
 #pragma unroll
   for (int s = 0; s < Z; s++) {
     const int tz = tz0 + s;
@@ -579,7 +575,7 @@ __global__ void __launch_bounds__(BX *BY)
     const float v = __fadd_rn((float)(tz + sz - nz / 2), (float)(nz / 2));
     const int vr = (int)(v - 1e-5f);
     float sum = 0.f;
-    if ((vr >= 0) & (vr < nz - 1)) sum = __fadd_rn(a[s], (v - vr) > 0.5f ? b[s] : b[s + 2]);
+    if ((vr >= 0) & (vr < nz - 1)) sum = __fmaf_rn(0.f, (v - vr) > 0.5f ? a[s] : a[s + 2], a[s + 1]);
     float *o = f + tx + (size_t)(n - ty - 1) * n + (size_t)tz * n * n;
     *o = __fmaf_rn(sum, c, *o);
   }
