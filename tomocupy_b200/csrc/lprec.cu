@@ -51,6 +51,7 @@ struct tcb_lprec {
   float *f32 = nullptr;   // fp32 output staging (FLOAT16 only)
   cudaArray_t ga = nullptr, fla = nullptr;
   cudaTextureObject_t texg = 0, texfl = 0;
+  cudaSurfaceObject_t surfg = 0, surffl = 0;  // the same arrays, as the kernels fill them
   cufftHandle fwd = 0, inv = 0;
   // own-FFT convolution
   bool own = false;
@@ -166,7 +167,9 @@ __global__ void prefilter_rows(float *__restrict__ g, int len, long long nlines)
 
 // The same along the angles of [nz][len][width]: blockDim.x neighbouring columns
 // of a slice per CTA (64-byte pieces of each row at 16), a thread per segment.
-__global__ void prefilter_cols(float *__restrict__ g, int width, int len) {
+// The coefficients also go into the layered array that the interpolation reads.
+__global__ void prefilter_cols(float *__restrict__ g, int width, int len,
+                               cudaSurfaceObject_t surf) {
   extern __shared__ float pf_sm[];
   const int st = pf_stride(len), c = threadIdx.x;
   const int x = blockIdx.x * blockDim.x + c;
@@ -178,8 +181,11 @@ __global__ void prefilter_cols(float *__restrict__ g, int width, int len) {
   __syncthreads();
   prefilter_line(pf_sm + c * st, len, threadIdx.y, on);
   if (on)
-    for (int k = threadIdx.y; k < len; k += blockDim.y)
-      base[(size_t)k * width] = pf_sm[c * st + pf_at(k)];
+    for (int k = threadIdx.y; k < len; k += blockDim.y) {
+      const float v = pf_sm[c * st + pf_at(k)];
+      base[(size_t)k * width] = v;
+      surf2DLayeredwrite(v, surf, x * (int)sizeof(float), k, blockIdx.y);
+    }
 }
 
 // Lines that are longer than a CTA's threads or shared memory hold: one thread
@@ -222,8 +228,20 @@ cudaError_t pf_attrs() {
   return e;
 }
 
-// Both passes over g [nz][nproj][n]: along the detector, then along the angles.
-int prefilter(float *g, int nz, int nproj, int n, cudaStream_t s) {
+int copy_to_array(cudaArray_t arr, const float *src, int w, int h, int d, cudaStream_t s) {
+  cudaMemcpy3DParms p = {};
+  p.srcPtr = make_cudaPitchedPtr((void *)src, w * sizeof(float), w, h);
+  p.dstArray = arr;
+  p.kind = cudaMemcpyDeviceToDevice;
+  p.extent = make_cudaExtent(w, h, d);
+  TCB_CUDA(cudaMemcpy3DAsync(&p, s));
+  return TCB_OK;
+}
+
+// Both passes over g [nz][nproj][n], along the detector, then along the angles,
+// and the result into the layered array.
+int prefilter(float *g, int nz, int nproj, int n, cudaArray_t arr, cudaSurfaceObject_t surf,
+              cudaStream_t s) {
   const long long nrows = (long long)nz * nproj;
   // as many lines per CTA as 512 threads (1024 along the angles) and 64 KB take
   auto lines = [](int len, int threads, int most) {
@@ -242,10 +260,11 @@ int prefilter(float *g, int nz, int nproj, int n, cudaStream_t s) {
   if (nproj <= PF_MAX) {
     const int l = lines(nproj, 1024, 16);
     prefilter_cols<<<dim3(ceil_div(n, l), nz), dim3(l, pf_nseg(nproj)),
-                     (size_t)l * pf_stride(nproj) * 4, s>>>(g, n, nproj);
+                     (size_t)l * pf_stride(nproj) * 4, s>>>(g, n, nproj, surf);
   } else {
     prefilter_serial<<<ceil_div((long long)nz * n, 128), 128, 0, s>>>(
         g, nproj, n, (long long)nz * n, n, (size_t)nproj * n, 1);
+    if (copy_to_array(arr, g, n, nproj, nz, s) != TCB_OK) return TCB_ERR_CUDA;
   }
   TCB_LAUNCH_CHECK();
   count_launch(2);
@@ -402,21 +421,19 @@ __global__ void __launch_bounds__(1024)
 }
 
 // Pass 3: row r: inverse FFT along theta, real part to slice 2q, imaginary
-// part to slice 2q + 1.
+// part to slice 2q + 1 of the layered array that the interpolation reads.
 template <int N>
 __global__ void __launch_bounds__(N / 16, (16384 / N < 16 ? 16384 / N : 16))
-    lc_rows_inv(const float2 *__restrict__ t2, float *__restrict__ fl,
+    lc_rows_inv(const float2 *__restrict__ t2, cudaSurfaceObject_t fl,
                 const float2 *__restrict__ tw, int nb, int nrho) {
   extern __shared__ float2 fsm[];
   const int r = blockIdx.x, q = blockIdx.y;
-  const size_t img = (size_t)nrho * N;
   const float2 *src = t2 + ((size_t)q * nrho + r) * N;
-  float *a = fl + (size_t)(2 * q) * img + (size_t)r * N;
-  float *b = 2 * q + 1 < nb ? a + img : nullptr;
+  const bool b = 2 * q + 1 < nb;
   auto in = [src](int e) { return __ldg(src + e); };
-  auto out = [a, b](int o, float2 v) {
-    a[o] = v.x;
-    if (b) b[o] = v.y;
+  auto out = [fl, b, r, q](int o, float2 v) {
+    surf2DLayeredwrite(v.x, fl, o * (int)sizeof(float), r, 2 * q);
+    if (b) surf2DLayeredwrite(v.y, fl, o * (int)sizeof(float), r, 2 * q + 1);
   };
   fftk::ifft<N>(fsm, threadIdx.x, tw, in, out);
 }
@@ -470,7 +487,7 @@ int lc_apply(tcb_lprec *h, cudaStream_t s) {
 #undef LC_COLS
   TCB_LAUNCH_CHECK();
 #define LC_INV(N)                                                                      \
-  lc_rows_inv<N><<<dim3((unsigned)nrho, pairs), N / 16, lc_rows_smem(N), s>>>(h->t2, h->fl, \
+  lc_rows_inv<N><<<dim3((unsigned)nrho, pairs), N / 16, lc_rows_smem(N), s>>>(h->t2, h->surffl, \
                                                                             h->twt, nb, nrho)
   LC_DISPATCH(ntheta, LC_INV)
 #undef LC_INV
@@ -481,21 +498,14 @@ int lc_apply(tcb_lprec *h, cudaStream_t s) {
 
 bool lc_pow2(int n) { return n >= 256 && n <= 8192 && (n & (n - 1)) == 0; }
 
-int copy_to_array(cudaArray_t arr, const float *src, int w, int h, int d, cudaStream_t s) {
-  cudaMemcpy3DParms p = {};
-  p.srcPtr = make_cudaPitchedPtr((void *)src, w * sizeof(float), w, h);
-  p.dstArray = arr;
-  p.kind = cudaMemcpyDeviceToDevice;
-  p.extent = make_cudaExtent(w, h, d);
-  TCB_CUDA(cudaMemcpy3DAsync(&p, s));
-  return TCB_OK;
-}
-
 void release(tcb_lprec *h) {
   if (h->fwd) cufftDestroy(h->fwd);
   if (h->inv) cufftDestroy(h->inv);
   if (h->texg) cudaDestroyTextureObject(h->texg);
   if (h->texfl) cudaDestroyTextureObject(h->texfl);
+  if (h->surfg) cudaDestroySurfaceObject(h->surfg);
+  if (h->surffl) cudaDestroySurfaceObject(h->surffl);
+  h->surfg = h->surffl = 0;
   if (h->ga) cudaFreeArray(h->ga);
   if (h->fla) cudaFreeArray(h->fla);
   cudaFree(h->fzs);
@@ -528,6 +538,14 @@ int make_tex(cudaArray_t arr, cudaTextureObject_t *tex) {
   td.normalizedCoords = 1;
   td.readMode = cudaReadModeElementType;
   TCB_CUDA(cudaCreateTextureObject(tex, &rd, &td, nullptr));
+  return TCB_OK;
+}
+
+int make_surf(cudaArray_t arr, cudaSurfaceObject_t *surf) {
+  cudaResourceDesc rd = {};
+  rd.resType = cudaResourceTypeArray;
+  rd.res.array.array = arr;
+  TCB_CUDA(cudaCreateSurfaceObject(surf, &rd));
   return TCB_OK;
 }
 
@@ -570,13 +588,13 @@ extern "C" int tcb_lprec_create(tcb_lprec **out, size_t nproj, size_t nz, size_t
        cudaMalloc(&h->f32, nz * n * n * sizeof(float)) != cudaSuccess))
     return fail(TCB_ERR_OUT_OF_MEMORY, "cudaMalloc failed");
   cudaChannelFormatDesc cd = cudaCreateChannelDesc<float>();
-  if (cudaMalloc3DArray(&h->ga, &cd, make_cudaExtent(n, nproj, nz), cudaArrayLayered) !=
-          cudaSuccess ||
-      cudaMalloc3DArray(&h->fla, &cd, make_cudaExtent(ntheta, nrho, nz), cudaArrayLayered) !=
-          cudaSuccess)
+  const unsigned aflags = cudaArrayLayered | cudaArraySurfaceLoadStore;
+  if (cudaMalloc3DArray(&h->ga, &cd, make_cudaExtent(n, nproj, nz), aflags) != cudaSuccess ||
+      cudaMalloc3DArray(&h->fla, &cd, make_cudaExtent(ntheta, nrho, nz), aflags) != cudaSuccess)
     return fail(TCB_ERR_OUT_OF_MEMORY, "cudaMalloc3DArray failed");
   if (pf_attrs() != cudaSuccess) return fail(TCB_ERR_CUDA, "shared-memory attribute failed");
-  if (make_tex(h->ga, &h->texg) != TCB_OK || make_tex(h->fla, &h->texfl) != TCB_OK)
+  if (make_tex(h->ga, &h->texg) != TCB_OK || make_tex(h->fla, &h->texfl) != TCB_OK ||
+      make_surf(h->ga, &h->surfg) != TCB_OK || make_surf(h->fla, &h->surffl) != TCB_OK)
     return fail(TCB_ERR_CUDA, nullptr);
   int dims[2] = {(int)nrho, (int)ntheta};
   int cemb[2] = {(int)nrho, (int)nc};
@@ -662,10 +680,9 @@ extern "C" int tcb_lprec_backprojection(tcb_lprec *h, void *f, void *g, void *st
   TCB_CUDA(cudaMemsetAsync(ff, 0, ftot * sizeof(float), s));
   {
     StageTimer st("lprec_prefilter", s);
-    const int rc = prefilter(gf, nz, nproj, n, s);
+    const int rc = prefilter(gf, nz, nproj, n, h->ga, h->surfg, s);
     if (rc != TCB_OK) return rc;
   }
-  if (copy_to_array(h->ga, gf, n, nproj, nz, s) != TCB_OK) return TCB_ERR_CUDA;
   TCB_CUFFT(cufftSetStream(h->fwd, s));
   TCB_CUFFT(cufftSetStream(h->inv, s));
   long long lpstep = (long long)ntheta * nrho;
@@ -700,8 +717,8 @@ extern "C" int tcb_lprec_backprojection(tcb_lprec *h, void *f, void *g, void *st
       TCB_LAUNCH_CHECK();
       count_launch();
       TCB_CUFFT(cufftExecC2R(h->inv, (cufftComplex *)h->flc, h->fl));
+      if (copy_to_array(h->fla, h->fl, ntheta, nrho, nz, s) != TCB_OK) return TCB_ERR_CUDA;
     }
-    if (copy_to_array(h->fla, h->fl, ntheta, nrho, nz, s) != TCB_OK) return TCB_ERR_CUDA;
     {
       StageTimer st("lprec_interp_c", s);
       dim3 g4(ceil_div(h->ncids, 256), nz);
