@@ -18,37 +18,74 @@ namespace {
 
 template <typename T> __device__ __forceinline__ float to_f32(T v) { return (float)v; }
 
-template <typename T>
-__global__ void darkflat_stats_kernel(float *__restrict__ dark0, float *__restrict__ flat0,
-                                      float *__restrict__ flat1,
-                                      const T *__restrict__ dark, const T *__restrict__ flat,
-                                      int ndark, int nflat, size_t plane, float bright_ratio,
-                                      int flat_linear) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// V neighbouring pixels per thread (16 bytes of frames), four frames in flight:
+// the frames are read once and HBM bounds it (10 darks and 10 flats of 2048^2
+// uint16: 0.065 ms; a pixel per thread with a division per flat took 0.187 ms).
+// Dividing by a bright ratio of 1 changes no value and is left out.
+template <typename T, int V>
+__global__ void __launch_bounds__(256)
+    darkflat_stats_kernel(float *__restrict__ dark0, float *__restrict__ flat0,
+                          float *__restrict__ flat1, const T *__restrict__ dark,
+                          const T *__restrict__ flat, int ndark, int nflat, size_t plane,
+                          float bright_ratio, int flat_linear) {
+  struct alignas(V * sizeof(T)) Px {
+    T v[V];
+  };
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (i >= plane) return;
+  const bool ratio = bright_ratio != 1.f;
+  // sum of frames k0 .. k1 - 1 in frame order, each divided by the bright ratio
+  auto sum = [&](const T *f, int k0, int k1, bool div, float (&s)[V]) {
+#pragma unroll
+    for (int e = 0; e < V; e++) s[e] = 0.f;
+#pragma unroll 4
+    for (int k = k0; k < k1; k++) {
+      const Px p = *reinterpret_cast<const Px *>(f + (size_t)k * plane + i);
+#pragma unroll
+      for (int e = 0; e < V; e++) {
+        const float x = to_f32(p.v[e]);
+        s[e] = __fadd_rn(s[e], div ? __fdiv_rn(x, bright_ratio) : x);
+      }
+    }
+  };
   // dark0 = mean(dark, axis=0): float32 sum in frame order, then / count.
-  float sd = 0.f;
-  for (int k = 0; k < ndark; k++) sd = __fadd_rn(sd, to_f32(dark[(size_t)k * plane + i]));
-  float d0 = __fdiv_rn(sd, (float)ndark);
-  dark0[i] = d0;
+  float d0[V], s[V];
+  sum(dark, 0, ndark, false, d0);
+#pragma unroll
+  for (int e = 0; e < V; e++) dark0[i + e] = d0[e] = __fdiv_rn(d0[e], (float)ndark);
   if (!flat_linear) {
-    float sf = 0.f;
-    for (int k = 0; k < nflat; k++)
-      sf = __fadd_rn(sf, __fdiv_rn(to_f32(flat[(size_t)k * plane + i]), bright_ratio));
-    float f0 = __fdiv_rn(sf, (float)nflat);
-    f0 = __fmul_rn(f0, 1.00001f);  // cp.float32(1 + 1e-5)
-    flat0[i] = __fsub_rn(f0, d0);
+    sum(flat, 0, nflat, ratio, s);
+#pragma unroll
+    for (int e = 0; e < V; e++) {
+      const float f0 = __fmul_rn(__fdiv_rn(s[e], (float)nflat), 1.00001f);  // cp.float32(1 + 1e-5)
+      flat0[i + e] = __fsub_rn(f0, d0[e]);
+    }
   } else {
     // flat0_p0 = mean(flat0[:nflat//2]), flat0_p1 = mean(flat0[nflat//2+1:])
-    int h = nflat / 2;
-    float s0 = 0.f, s1 = 0.f;
-    for (int k = 0; k < h; k++)
-      s0 = __fadd_rn(s0, __fdiv_rn(to_f32(flat[(size_t)k * plane + i]), bright_ratio));
-    for (int k = h + 1; k < nflat; k++)
-      s1 = __fadd_rn(s1, __fdiv_rn(to_f32(flat[(size_t)k * plane + i]), bright_ratio));
-    flat0[i] = __fdiv_rn(s0, (float)h);
-    flat1[i] = __fdiv_rn(s1, (float)(nflat - h - 1));
+    const int h = nflat / 2;
+    sum(flat, 0, h, ratio, s);
+#pragma unroll
+    for (int e = 0; e < V; e++) flat0[i + e] = __fdiv_rn(s[e], (float)h);
+    sum(flat, h + 1, nflat, ratio, s);
+#pragma unroll
+    for (int e = 0; e < V; e++) flat1[i + e] = __fdiv_rn(s[e], (float)(nflat - h - 1));
   }
+}
+
+// Vectors of 16 bytes of frames where every frame starts on one, else single pixels.
+template <typename T>
+void launch_stats(float *dark0, float *flat0, float *flat1, const void *dark, const void *flat,
+                  int ndark, int nflat, size_t plane, float bright_ratio, int flat_linear,
+                  cudaStream_t s) {
+  constexpr int V = 16 / sizeof(T);
+  if (plane % V == 0 && (((uintptr_t)dark | (uintptr_t)flat) & 15) == 0)
+    darkflat_stats_kernel<T, V><<<ceil_div(plane / V, 256), 256, 0, s>>>(
+        dark0, flat0, flat1, (const T *)dark, (const T *)flat, ndark, nflat, plane, bright_ratio,
+        flat_linear);
+  else
+    darkflat_stats_kernel<T, 1><<<ceil_div(plane, 256), 256, 0, s>>>(
+        dark0, flat0, flat1, (const T *)dark, (const T *)flat, ndark, nflat, plane, bright_ratio,
+        flat_linear);
 }
 
 struct PrepArgs {
@@ -220,24 +257,20 @@ extern "C" int tcb_darkflat_stats(void *dark0, void *flat0, void *flat1, const v
   size_t plane = nz * n;
   if (plane == 0) return TCB_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned grid = ceil_div(plane, 256);
   StageTimer st("darkflat_stats", s);
   count_launch();
   switch (in_dtype) {
     case TCB_U16:
-      darkflat_stats_kernel<uint16_t><<<grid, 256, 0, s>>>(
-          (float *)dark0, (float *)flat0, (float *)flat1, (const uint16_t *)dark,
-          (const uint16_t *)flat, (int)ndark, (int)nflat, plane, bright_ratio, flat_linear);
+      launch_stats<uint16_t>((float *)dark0, (float *)flat0, (float *)flat1, dark, flat, (int)ndark,
+                         (int)nflat, plane, bright_ratio, flat_linear, s);
       break;
     case TCB_U8:
-      darkflat_stats_kernel<uint8_t><<<grid, 256, 0, s>>>(
-          (float *)dark0, (float *)flat0, (float *)flat1, (const uint8_t *)dark,
-          (const uint8_t *)flat, (int)ndark, (int)nflat, plane, bright_ratio, flat_linear);
+      launch_stats<uint8_t>((float *)dark0, (float *)flat0, (float *)flat1, dark, flat, (int)ndark,
+                         (int)nflat, plane, bright_ratio, flat_linear, s);
       break;
     case TCB_F32:
-      darkflat_stats_kernel<float><<<grid, 256, 0, s>>>(
-          (float *)dark0, (float *)flat0, (float *)flat1, (const float *)dark,
-          (const float *)flat, (int)ndark, (int)nflat, plane, bright_ratio, flat_linear);
+      launch_stats<float>((float *)dark0, (float *)flat0, (float *)flat1, dark, flat, (int)ndark,
+                         (int)nflat, plane, bright_ratio, flat_linear, s);
       break;
     default:
       set_error("tcb_darkflat_stats: unknown dtype %d", in_dtype);
@@ -389,7 +422,6 @@ extern "C" int tcb_prep_noalloc(float *out, const void *data, const void *dark,
   float *dark0 = stats, *flat0 = stats + TCB_NOALLOC_MAX_PLANE;
   size_t plane = nz * n;
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned sgrid = ceil_div(plane, 256);
   PrepArgs a{out, nullptr, nullptr, data, dark0, flat0, nullptr, (int)nproj, (int)nz, (int)n,
              nz * n, n, out_zstride, out_pstride, out_poff, out_xoff, out_width,
              flags | TCB_PREP_DARKFLAT};
@@ -397,23 +429,20 @@ extern "C" int tcb_prep_noalloc(float *out, const void *data, const void *dark,
   StageTimer t("prep_noalloc", s);
   switch (in_dtype) {
     case TCB_U16:
-      darkflat_stats_kernel<uint16_t><<<sgrid, 256, 0, s>>>(
-          dark0, flat0, nullptr, (const uint16_t *)dark, (const uint16_t *)flat, (int)ndark,
-          (int)nflat, plane, bright_ratio, 0);
+      launch_stats<uint16_t>(dark0, flat0, nullptr, dark, flat, (int)ndark, (int)nflat, plane, bright_ratio,
+                         0, s);
       TCB_LAUNCH_CHECK();
       prep_rows_kernel<uint16_t, false><<<prep_grid(rows), 256, 0, s>>>(a);
       break;
     case TCB_U8:
-      darkflat_stats_kernel<uint8_t><<<sgrid, 256, 0, s>>>(
-          dark0, flat0, nullptr, (const uint8_t *)dark, (const uint8_t *)flat, (int)ndark,
-          (int)nflat, plane, bright_ratio, 0);
+      launch_stats<uint8_t>(dark0, flat0, nullptr, dark, flat, (int)ndark, (int)nflat, plane, bright_ratio,
+                         0, s);
       TCB_LAUNCH_CHECK();
       prep_rows_kernel<uint8_t, false><<<prep_grid(rows), 256, 0, s>>>(a);
       break;
     default:
-      darkflat_stats_kernel<float><<<sgrid, 256, 0, s>>>(
-          dark0, flat0, nullptr, (const float *)dark, (const float *)flat, (int)ndark,
-          (int)nflat, plane, bright_ratio, 0);
+      launch_stats<float>(dark0, flat0, nullptr, dark, flat, (int)ndark, (int)nflat, plane, bright_ratio,
+                         0, s);
       TCB_LAUNCH_CHECK();
       prep_rows_kernel<float, false><<<prep_grid(rows), 256, 0, s>>>(a);
   }
