@@ -51,6 +51,7 @@ constexpr int VO_MAXW = 127;   // largest median window
 
 __device__ __forceinline__ int reflect_idx(int i, int n) {
   // scipy.ndimage mode 'reflect' (d c b a | a b c d | d c b a)
+  if ((unsigned)i < (unsigned)n) return i;
   const int p = 2 * n;
   int m = i % p;
   if (m < 0) m += p;
@@ -183,7 +184,11 @@ void sort_columns(const float *tt, int nproj, int ni, int nz, float *srt, int *i
 
 // Median over w (odd) columns, reflect mode, of in[(z * ni + x) * R + r] for
 // every (z, x, r): each thread slides a sorted window along a run of VO_RUN
-// columns of one (z, r) (window kept interleaved in shared memory).
+// columns of one (z, r) (window kept interleaved in shared memory).  A chain of
+// dependent shared-memory loads bounds it, so the places of the leaving and of
+// the entering value are searched for together and the values between them move
+// four at a time (one by one, after one search: 1.08 ms for windows of 61 and 21
+// on 16 x 720 x 1024; so 0.58).
 __global__ void __launch_bounds__(VO_MED_T)
     vo_median_x(const float *__restrict__ in, float *__restrict__ out, int nz, int ni, int R,
                 int w) {
@@ -210,25 +215,35 @@ __global__ void __launch_bounds__(VO_MED_T)
   out[((size_t)z * ni + x0) * R + r] = W(h);
   for (int x = x0 + 1; x < x1; x++) {
     const float vo = val(x - h - 1), vn = val(x + h);
-    int lo = 0, hi = w - 1;  // first position holding a value >= vo (vo is present)
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (W(mid) < vo) lo = mid + 1; else hi = mid;
+    // first places of values >= vo (vo is among them) and >= vn, side by side
+    int lo = 0, hi = w, pl = 0, ph = w;
+    while (lo < hi || pl < ph) {
+      const int m = min((lo + hi) >> 1, w - 1), q = min((pl + ph) >> 1, w - 1);
+      const float a = W(m), b = W(q);
+      if (lo < hi) {
+        if (a < vo) lo = m + 1; else hi = m;
+      }
+      if (pl < ph) {
+        if (b < vn) pl = q + 1; else ph = q;
+      }
     }
+    lo = min(lo, w - 1);
+    // the values between move by one, four loads ahead of their stores
     int i = lo;
+    if (vn > vo) {
+      for (; i + 4 < pl; i += 4) {
+        const float a = W(i + 1), b = W(i + 2), c = W(i + 3), d = W(i + 4);
+        W(i) = a, W(i + 1) = b, W(i + 2) = c, W(i + 3) = d;
+      }
+      for (; i + 1 < pl; i++) W(i) = W(i + 1);
+    } else {
+      for (; i - 4 >= pl; i -= 4) {
+        const float a = W(i - 1), b = W(i - 2), c = W(i - 3), d = W(i - 4);
+        W(i) = a, W(i - 1) = b, W(i - 2) = c, W(i - 3) = d;
+      }
+      for (; i > pl; i--) W(i) = W(i - 1);
+    }
     W(i) = vn;
-    while (i + 1 < w && W(i + 1) < W(i)) {
-      const float a = W(i);
-      W(i) = W(i + 1);
-      W(i + 1) = a;
-      i++;
-    }
-    while (i > 0 && W(i - 1) > W(i)) {
-      const float a = W(i);
-      W(i) = W(i - 1);
-      W(i - 1) = a;
-      i--;
-    }
     out[((size_t)z * ni + x) * R + r] = W(h);
   }
 }
