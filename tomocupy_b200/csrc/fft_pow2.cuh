@@ -124,6 +124,19 @@ template <int N> struct Plan {
   static constexpr int T = N / 16;                             // threads per transform
   static constexpr int PADDED = N + N / 16;                    // smem slots per transform
 };
+
+// Transforms side by side in one block (column passes): as many as fill 1024
+// threads, at most 16, and the shared-memory stride between them, 16 / count
+// slots beyond the padded length: the lanes of a half-warp (a few consecutive
+// threads of each transform) then fall on different banks.  (A stride of
+// PADDED + 4 for every N made half of the accesses conflict at 8 x 2048.)
+__host__ __device__ constexpr int columns_per_block(int n) {
+  return 16384 / n < 16 ? 16384 / n : 16;
+}
+__host__ __device__ constexpr int column_stride(int n) {
+  return n + n / 16 + 16 / columns_per_block(n);
+}
+
 template <int N, int S> constexpr int radix_of() {
   return S < Plan<N>::NS16 ? 16 : Plan<N>::RL;
 }

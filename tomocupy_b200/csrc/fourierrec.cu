@@ -1508,7 +1508,7 @@ __global__ void __launch_bounds__(1024) ifft_cols(const float2 *__restrict__ gri
                                                  float2 *__restrict__ t1,
                                                  const float2 *__restrict__ tw, int cpc) {
   extern __shared__ float2 fsm[];
-  constexpr int SSTR = fftk::Plan<N>::PADDED + 4;
+  constexpr int SSTR = fftk::column_stride(N);
   const int c = threadIdx.x % cpc, tid = threadIdx.x / cpc;
   const int ncb = N / cpc;
   const int z = blockIdx.x / ncb, x = (blockIdx.x % ncb) * cpc + c;
@@ -1617,7 +1617,7 @@ __global__ void __launch_bounds__(1024) ifft_cols_deapod(const float2 *__restric
                                                          Geom geo, int unpack, int cpc) {
   extern __shared__ float2 fsm[];
   constexpr int n = N / 2;
-  constexpr int SSTR = fftk::Plan<N>::PADDED + 4;
+  constexpr int SSTR = fftk::column_stride(N);
   const int c = threadIdx.x % cpc, tid = threadIdx.x / cpc;
   const int ncb = n / cpc;
   const int z = blockIdx.x / ncb, tx = (blockIdx.x % ncb) * cpc + c;
@@ -1636,7 +1636,7 @@ __global__ void __launch_bounds__(1024) ifft_cols_deapod(const float2 *__restric
 }
 
 inline int cols_per_block(int N) { return std::min(16384 / N, 16); }
-inline size_t cols_smem(int N, int cpc) { return (size_t)cpc * (N + N / 16 + 4) * sizeof(float2); }
+inline size_t cols_smem(int N, int cpc) { return (size_t)cpc * fftk::column_stride(N) * sizeof(float2); }
 inline size_t rows_smem(int N) { return (size_t)(N + N / 16) * sizeof(float2); }
 
 template <int N, int GW>

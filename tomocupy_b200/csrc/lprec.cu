@@ -149,7 +149,15 @@ __host__ __device__ inline int pf_stride(int len) { return (pf_at(len - 1) + 1) 
 // CTA, a thread per segment, HBM read and written once.  Along a whole line per
 // lane (900 warps on the chip for 32 x 900 lines) and, for the angles, a whole
 // column per thread, the two passes took 1.12 ms at 32 x 900 x 1024, serial
-// chains all; these two take 0.28 ms (the HBM traffic alone 0.07).
+// chains all; these two take 0.21 ms (the HBM traffic alone 0.07).
+__device__ __forceinline__ void pf_fetch(float *dst, const float *src) {  // asynchronously
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void pf_fetched() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __global__ void prefilter_rows(float *__restrict__ g, int len, long long nlines) {
   extern __shared__ float pf_sm[];
   const int lines = blockDim.y, st = pf_stride(len);
@@ -158,7 +166,8 @@ __global__ void prefilter_rows(float *__restrict__ g, int len, long long nlines)
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
   float *base = g + l0 * len;
   for (int l = 0; l < nl; l++)
-    for (int k = tid; k < len; k += nt) pf_sm[l * st + pf_at(k)] = base[(size_t)l * len + k];
+    for (int k = tid; k < len; k += nt) pf_fetch(pf_sm + l * st + pf_at(k), base + (size_t)l * len + k);
+  pf_fetched();
   __syncthreads();
   prefilter_line(pf_sm + threadIdx.y * st, len, threadIdx.x, (int)threadIdx.y < nl);
   for (int l = 0; l < nl; l++)
@@ -177,7 +186,8 @@ __global__ void prefilter_cols(float *__restrict__ g, int width, int len,
   float *base = g + (size_t)blockIdx.y * width * len + x;
   if (on)
     for (int k = threadIdx.y; k < len; k += blockDim.y)
-      pf_sm[c * st + pf_at(k)] = base[(size_t)k * width];
+      pf_fetch(pf_sm + c * st + pf_at(k), base + (size_t)k * width);
+  pf_fetched();
   __syncthreads();
   prefilter_line(pf_sm + c * st, len, threadIdx.y, on);
   if (on)
@@ -381,7 +391,7 @@ __global__ void __launch_bounds__(1024)
             const float2 *__restrict__ fzs, const float2 *__restrict__ h0,
             const float2 *__restrict__ tw, int ntheta, int cpc) {
   extern __shared__ float2 fsm[];
-  constexpr int SSTR = fftk::Plan<N>::PADDED + 4;
+  constexpr int SSTR = fftk::column_stride(N);
   const int c = threadIdx.x % cpc, tid = threadIdx.x / cpc;
   const int ncb = ntheta / cpc;
   const int q = blockIdx.x / ncb, j = (blockIdx.x % ncb) * cpc + c;
@@ -439,7 +449,7 @@ __global__ void __launch_bounds__(N / 16, (16384 / N < 16 ? 16384 / N : 16))
 }
 
 inline int lc_cpc(int N) { return std::min(16384 / N, 16); }
-inline size_t lc_cols_smem(int N) { return (size_t)lc_cpc(N) * (N + N / 16 + 4) * sizeof(float2); }
+inline size_t lc_cols_smem(int N) { return (size_t)lc_cpc(N) * fftk::column_stride(N) * sizeof(float2); }
 inline size_t lc_rows_smem(int N) { return (size_t)(N + N / 16) * sizeof(float2); }
 
 #define LC_DISPATCH(n, F)      \

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(1024)
     ph_cols(const float2 *__restrict__ t1, float2 *__restrict__ t2, const float *__restrict__ fe,
             const float2 *__restrict__ tw, int Nz, int dy, int py, int cpc) {
   extern __shared__ float2 fsm[];
-  constexpr int SSTR = fftk::Plan<N>::PADDED + 4;
+  constexpr int SSTR = fftk::column_stride(N);
   const int c = threadIdx.x % cpc, tid = threadIdx.x / cpc;
   const int ncb = Nz / cpc;
   const int q = blockIdx.x / ncb, j = (blockIdx.x % ncb) * cpc + c;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(N / 16, (16384 / N < 16 ? 16384 / N : 16))
 }
 
 inline int ph_cpc(int N) { return std::min(16384 / N, 16); }
-inline size_t ph_cols_smem(int N) { return (size_t)ph_cpc(N) * (N + N / 16 + 4) * sizeof(float2); }
+inline size_t ph_cols_smem(int N) { return (size_t)ph_cpc(N) * fftk::column_stride(N) * sizeof(float2); }
 inline size_t ph_rows_smem(int N) { return (size_t)(N + N / 16) * sizeof(float2); }
 
 template <int N>
