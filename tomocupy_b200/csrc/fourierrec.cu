@@ -1030,18 +1030,25 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 
 // Warp roles of the streamed-weight gridding: 16 accumulator warps (warp w
 // reads TMEM lanes 32 (w % 4) .. of M-group (w / 4) % 2, columns half w / 8),
-// one producer warp (bulk copies of W, cp.async gathers of V) and one warp
-// whose lane 0 issues the MMAs.
+// one or two producer warps (bulk copies of W, cp.async gathers of V) and one
+// warp whose lane 0 issues the MMAs.
 constexpr int WS_ACC_WARPS = 16;
-constexpr int WS_THREADS = (WS_ACC_WARPS + 2) * 32;
 
 template <int NN, bool SPLIT>
 struct SwCfg {
   static constexpr int NST = SPLIT ? 4 : 8;                  // shared-memory stages
+  // producer warps: chunk g of a CTA is warp g % PROD's.  One warp's instructions
+  // take longer than a chunk's bytes, except where those are most (two against
+  // one: mixed 1024 x 720 x 32 pairs 0.33 and 0.41 ms, fp32 0.54 and 0.56; fp32
+  // 2048 x 1500 x 64 pairs 3.20 and 2.89, where two warps keep one chunk each
+  // unpublished in a ring of four, one keeps two)
+  static constexpr int PROD = SPLIT && NN == 128 ? 1 : 2;
+  static constexpr int THREADS = (WS_ACC_WARPS + PROD + 1) * 32;
   // a chunk's gathers are published (fenced, then arrived on its stage's
-  // mbarrier) once LAG newer chunks have been issued: the producer lanes wait
-  // for their cp.async groups LAG deep instead of one chunk at a time
-  static constexpr int LAG = NST / 2;
+  // mbarrier) once its producer warp has issued LAG newer chunks: the lanes wait
+  // for their cp.async groups LAG deep instead of one chunk at a time.  A warp's
+  // unpublished chunks must not fill the ring: PROD (LAG + 1) <= NST
+  static constexpr int LAG = NST / PROD - 1 < 2 ? NST / PROD - 1 : 2;
   static constexpr int WB = SPLIT ? 2 * SW_WIMG : SW_WIMG;   // W bytes per stage
   static constexpr int VB = SW_K * NN * 2;                   // one V operand
   static constexpr int STAGE = WB + (SPLIT ? 2 : 1) * VB;
@@ -1100,7 +1107,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
 // then give up at their next wait, and the CTA lets its copies and MMAs in
 // flight finish (bounded) before it frees TMEM.
 template <int NN, bool SPLIT>
-__global__ void __launch_bounds__(WS_THREADS, 1)
+__global__ void __launch_bounds__(SwCfg<NN, SPLIT>::THREADS, 1)
     grid_sw(const uint4 *__restrict__ whi, const uint4 *__restrict__ wlo,
             const int *__restrict__ vidx, const int2 *__restrict__ tile_chunks,
             const int *__restrict__ tile_order, int ntiles, int nitems,
@@ -1110,7 +1117,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
             int *__restrict__ err) {
   using namespace tcb::tc;
   using Cfg = SwCfg<NN, SPLIT>;
-  constexpr int NST = Cfg::NST;
+  constexpr int NST = Cfg::NST, PROD = Cfg::PROD;
   // fp16 grid (tscale != null): per-warp maxima of each pair over a tile, two
   // item parities x two column halves x 8 warps
   __shared__ float s_red[2][2][8][32];
@@ -1144,15 +1151,17 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
   bool ok = true;
 
-  if (warp == WS_ACC_WARPS) {
-    // ---------------- producer
-    long long g = 0;      // chunks issued
-    long long pub = 0;    // chunks whose gathers this lane has published
+  if (warp >= WS_ACC_WARPS && warp < WS_ACC_WARPS + PROD) {
+    // ---------------- producers
+    const int me = warp - WS_ACC_WARPS;
+    long long g = 0;      // chunks of the CTA passed
+    long long own = 0;    // chunks issued by this warp: me, me + PROD, ..
+    long long pub = 0;    // of those, chunks whose gathers this lane has published
     int it = blockIdx.x;
     int2 cur = it < nitems ? tile_chunks[tile_order[it % ntiles]] : make_int2(0, 0);
     int tnext = it + G < nitems ? tile_order[(it + G) % ntiles] : 0;
-    int row = cur.y > 0 ? __ldg(vidx + (size_t)cur.x * SW_K + lane) : -1;
-    bool have_row = true;
+    int row = cur.y > me ? __ldg(vidx + (size_t)(cur.x + me) * SW_K + lane) : -1;
+    bool have_row = cur.y > me;
     for (; it < nitems && ok; it += G) {
       // one item ahead: the next item's chunk range, the tile of the one after
       const int2 nxt = it + G < nitems ? tile_chunks[tnext] : make_int2(0, 0);
@@ -1160,15 +1169,19 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
       const int zg = it / ntiles;
       const __half *gh = ghi + (size_t)zg * rows * NN;
       const __half *gl = SPLIT ? glo + (size_t)zg * rows * NN : nullptr;
-      if (cur.y > 0 && !have_row) row = __ldg(vidx + (size_t)cur.x * SW_K + lane);
-      have_row = false;
-      for (int c = 0; c < cur.y; c++, g++) {
-        // the row index of the chunk after this one (possibly the next item's first)
+      // this warp's first chunk of the item
+      int c = (int)((me - g % PROD + PROD) % PROD);
+      const long long g0 = g;
+      if (cur.y > c && !have_row) row = __ldg(vidx + (size_t)(cur.x + c) * SW_K + lane);
+      if (cur.y > c) have_row = false;
+      for (; c < cur.y; c += PROD, own++) {
+        g = g0 + c;
+        // the row index of this warp's next chunk (possibly in the next item)
         int row_next = -1;
-        if (c + 1 < cur.y) {
-          row_next = __ldg(vidx + (size_t)(cur.x + c + 1) * SW_K + lane);
-        } else if (nxt.y > 0) {
-          row_next = __ldg(vidx + (size_t)nxt.x * SW_K + lane);
+        if (c + PROD < cur.y) {
+          row_next = __ldg(vidx + (size_t)(cur.x + c + PROD) * SW_K + lane);
+        } else if (nxt.y > c + PROD - cur.y) {
+          row_next = __ldg(vidx + (size_t)(nxt.x + c + PROD - cur.y) * SW_K + lane);
           have_row = true;
         }
         const int s = (int)(g % NST);
@@ -1203,25 +1216,26 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
           if (SPLIT) cp_async16(vb + Cfg::VB + d, gl + so, nb);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        // chunk g - LAG's gathers have landed: publish them to the async proxy
-        if (g + 1 - pub > Cfg::LAG) {
+        // the gathers of LAG chunks ago have landed: publish them to the async proxy
+        if (own + 1 - pub > Cfg::LAG) {
           asm volatile("cp.async.wait_group %0;" ::"n"(Cfg::LAG) : "memory");
           fence_proxy_async_smem();
-          mbar_arrive(&full[pub % NST]);
+          mbar_arrive(&full[(me + PROD * pub) % NST]);
           pub++;
         }
         row = row_next;
       }
+      g = g0 + cur.y;
       cur = nxt;
       tnext = tnext2;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     fence_proxy_async_smem();
-    for (; pub < g; pub++) mbar_arrive(&full[pub % NST]);
+    for (; pub < own; pub++) mbar_arrive(&full[(me + PROD * pub) % NST]);
     // the bulk copies of the last stages have landed before the CTA exits (bounded)
-    for (long long gg = g > NST ? g - NST : 0; gg < g; gg++)
-      mbar_wait(&full[gg % NST], (uint32_t)((gg / NST) & 1));
-  } else if (warp == WS_ACC_WARPS + 1) {
+    for (long long k = own > NST / PROD ? own - NST / PROD : 0; k < own; k++)
+      mbar_wait(&full[(me + PROD * k) % NST], (uint32_t)(((me + PROD * k) / NST) & 1));
+  } else if (warp == WS_ACC_WARPS + PROD) {
     // ---------------- MMA issuer
     long long g = 0, gp = 0;  // chunks consumed, TMEM buffers started
     int it = blockIdx.x;
@@ -1991,7 +2005,7 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
     const int nitems = h->sw_ntiles * h->sw_zgroups;
     const unsigned grd = (unsigned)std::min(nitems, sm_count());
 #define FR_SW(NN_, SPLIT_)                                                                 \
-  grid_sw<NN_, SPLIT_><<<grd, WS_THREADS, SwCfg<NN_, SPLIT_>::SMEM, s>>>(                  \
+  grid_sw<NN_, SPLIT_><<<grd, SwCfg<NN_, SPLIT_>::THREADS, SwCfg<NN_, SPLIT_>::SMEM, s>>>( \
       h->sw_whi, h->sw_wlo, h->sw_vidx, h->sw_tile_chunks, h->sw_order, h->sw_ntiles,       \
       nitems, h->sw_ghi, h->sw_glo, h->amax, h->grid, geo, h->sw_ntx, rows, skip ? 1 : 0,   \
       grid_h ? h->sw_tscale : nullptr, h->tc_err)
