@@ -174,16 +174,18 @@ class SinoPipeline:
                           if self.out_dtype == torch.float16 else None)
 
     def _set_gridding(self, gridding: str, precision: str) -> int:
-        """fourierrec gridding mode.  'auto': up to 16 slice pairs per chunk
-        (8 in mixed precision) the fp32 register gridding, which needs no weight
-        tables and is the faster there (16 pairs, against split-fp16 weights:
-        0.56 and 0.65 ms at 1024 x 720, 2.28 and 2.35 ms at 2048 x 1500; 24
-        pairs: 0.83 and 0.72 ms, 3.41 and 2.60 ms; 8 pairs, against fp16 weights:
-        0.29 and 0.50 ms, 1.15 and 1.73 ms; 16 pairs: 0.56 and 0.53 ms, 2.28 and
-        1.86 ms); above that the tensor cores with streamed weights (split fp16
+        """fourierrec gridding mode.  'auto': up to 8 slice pairs per chunk the
+        fp32 register gridding, which needs no weight tables and is the faster
+        there (8 pairs, against split-fp16 weights: 0.29 and 0.50 ms at 1024 x 720,
+        1.15 and 1.78 ms at 2048 x 1500; against fp16 weights, mixed precision:
+        0.29 and 0.35, 1.15 and 1.24 ms), in float32 up to 16 where angles x columns
+        are at most 2^20, whose fewer tiles leave the tensor cores waiting for the
+        centre's (16 pairs: 0.15 and 0.20 ms at 512 x 360, 0.29 and 0.35 at
+        768 x 500, 0.56 and 0.55 at 1024 x 720, but 2.28 and 2.01 at
+        2048 x 1500); above that the tensor cores with streamed weights (split fp16
         for float32, fp16 for mixed) when their tables fit in device memory, else
-        the register gridding (float32) or the tensor-core gridding that builds
-        its weights per chunk (mixed).
+        the register gridding (float32) or the tensor-core gridding that builds its
+        weights per chunk (mixed).
         'fp32' / 'tensor' / 'tensor_fp32' / 'tensor_stream' force a mode."""
         modes = {"fp32": _lib.GRID_FP32, "tensor": _lib.GRID_TENSOR,
                  "tensor_fp32": _lib.GRID_TENSOR_FP32, "tensor_stream": _lib.GRID_TENSOR_STREAM}
@@ -193,7 +195,8 @@ class SinoPipeline:
         first = _lib.GRID_TENSOR_STREAM if precision == "mixed" else _lib.GRID_TENSOR_FP32
         if os.environ.get("TCB_FOURIERREC_GRIDDING") in modes:
             first = modes[os.environ["TCB_FOURIERREC_GRIDDING"]]
-        elif self.ncz // 2 <= (8 if precision == "mixed" else 16):
+        elif self.ncz // 2 <= (16 if precision == "float32" and
+                               self.n * self.nproj <= 1 << 20 else 8):
             first = _lib.GRID_FP32
         fallback = _lib.GRID_TENSOR if precision == "mixed" else _lib.GRID_FP32
         try:
