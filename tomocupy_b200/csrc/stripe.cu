@@ -205,256 +205,360 @@ __global__ void sfb_rows(const float *__restrict__ in, int H, int Wi, float *__r
 }
 
 // ---- register-blocked filter banks for the supported filter lengths ------
-// Same outputs, bit for bit, as the kernels above (every output keeps its
-// multiply-then-add tap order); the taps come from the kernel parameter
-// space (constant-bank operands of the multiplies, fully unrolled), and each
-// input value is read once per thread window instead of once per tap.
+// Same outputs, bit for bit, as the kernels above: every output keeps its
+// multiply-then-add tap order, two outputs at a time in the halves of packed
+// f32x2 instructions (two rows of the last axis, two columns of the other), so
+// a tap costs one packed multiply and one packed add for both.  The multiply is
+// a fused multiply-add of -0, which rounds as a multiply does and, unlike a
+// packed multiply, cannot be contracted with the add that follows; the zero
+// comes with the taps so that the compiler does not know it.
+// These instructions (two cycles of the FP32 pipe each) are the bound: 0.13 ms per
+// pass over the 7 levels of 16 slices of 1500 x 2048 at 32 taps.  Measured there,
+// one output at a time and packed: analysis rows 0.45 and 0.44 ms, columns 0.40
+// and 0.36, synthesis columns 0.51 and 0.36, rows 0.41 and 0.40; what is left is
+// the staging's latency (rows) and the few warps 127 registers leave (columns).
 struct TapPair {
-  float a[MAXL], b[MAXL];
+  float4 c[MAXL];  // (a, a, b, b) of tap k
+  float2 nz;       // -0, -0
 };
 
-// afb1d along the last axis.  RB rows per block staged in shared memory with
-// the symmetric extension applied (smem[u] = x[reflect(u - padl)]); output j
-// reads smem[2j + k], k < L, as L/2 float2 loads (conflict-free).
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b, f32x2 nz) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// The taps in shared memory, as one 16-byte broadcast per tap: the packed
+// instructions take them from registers only, and a pair from the constant bank
+// costs several moves.
 template <int L>
-__global__ void __launch_bounds__(256) afb_rows_t(const float *__restrict__ x, long long sz,
-                                                  int sx, float *__restrict__ out, int B, int H,
-                                                  int W, int Wo, int padl, int RB, int SW,
-                                                  const __grid_constant__ TapPair t) {
-  extern __shared__ float2 srow2[];
-  float *srow = reinterpret_cast<float *>(srow2);
-  const long long row0 = (long long)blockIdx.x * RB;
-  const long long nrows = (long long)B * H;
-  const int nr = (int)min((long long)RB, nrows - row0);
-  for (int r = 0; r < nr; r++) {
-    const long long row = row0 + r;
-    const long long b = row / H, h = row - b * H;
-    const float *xr = x + b * sz + h * sx;
-    float *sr = srow + r * SW;
-    for (int u = threadIdx.x; u < SW; u += blockDim.x) {
-      const int m = u - padl;
-      sr[u] = xr[m >= 0 && m < W ? m : reflect(m, W)];
-    }
-  }
-  __syncthreads();
-  constexpr int RO = 4;                 // outputs per thread
-  constexpr int NV = 2 * RO + L - 2;    // their input window
-  const int ngrp = (Wo + RO - 1) / RO;
-  for (int e = threadIdx.x; e < nr * ngrp; e += blockDim.x) {
-    const int r = e / ngrp, j0 = (e - r * ngrp) * RO;
-    const float2 *p = srow2 + (r * SW) / 2 + j0;  // smem[2 j0 + u] = window u
-    float v[NV];
+__device__ __forceinline__ f32x2 stage_taps(ulonglong2 (&st)[L], const TapPair &t) {
+  for (int k = threadIdx.x; k < L; k += blockDim.x)
+    st[k] = make_ulonglong2(pack2(t.c[k].x, t.c[k].y), pack2(t.c[k].z, t.c[k].w));
+  return pack2(t.nz.x, t.nz.y);
+}
+
+// Analysis: lo/hi[o] = sum over k of the taps times win(2 o + k), o < RO.
+template <int L, int RO, class Win>
+__device__ __forceinline__ void analyse(const ulonglong2 *taps, f32x2 nz, Win win,
+                                        f32x2 (&lo)[RO], f32x2 (&hi)[RO]) {
+  f32x2 v[2 * RO + L - 2];
 #pragma unroll
-    for (int q = 0; q < NV / 2; q++) {
-      const float2 w = p[q];
-      v[2 * q] = w.x;
-      v[2 * q + 1] = w.y;
-    }
-    float lo[RO], hi[RO];
+  for (int q = 0; q < 2 * RO - 2; q++) v[q] = win(q);
+#pragma unroll
+  for (int k = 0; k < L; k++) {
+    v[2 * RO - 2 + k] = win(2 * RO - 2 + k);
+    const ulonglong2 c = taps[k];
 #pragma unroll
     for (int o = 0; o < RO; o++) {
-      lo[o] = __fmul_rn(t.a[0], v[2 * o]);
-      hi[o] = __fmul_rn(t.b[0], v[2 * o]);
+      const f32x2 x = mul2(c.x, v[2 * o + k], nz), y = mul2(c.y, v[2 * o + k], nz);
+      lo[o] = k ? add2(lo[o], x) : x;
+      hi[o] = k ? add2(hi[o], y) : y;
     }
-#pragma unroll
-    for (int k = 1; k < L; k++) {
-      const float ak = t.a[k], bk = t.b[k];
-#pragma unroll
-      for (int o = 0; o < RO; o++) {
-        lo[o] = __fadd_rn(lo[o], __fmul_rn(ak, v[2 * o + k]));
-        hi[o] = __fadd_rn(hi[o], __fmul_rn(bk, v[2 * o + k]));
-      }
-    }
-    const long long row = row0 + r;
-    const long long b = row / H, h = row - b * H;
-    float *o0 = out + ((b * 2) * H + h) * Wo;
-    float *o1 = o0 + (long long)H * Wo;
-#pragma unroll
-    for (int o = 0; o < RO; o++)
-      if (j0 + o < Wo) {
-        o0[j0 + o] = lo[o];
-        o1[j0 + o] = hi[o];
-      }
   }
 }
 
-// Column kernels: a block is a tile of 32 columns x (8 * RO) output rows of
-// one channel plane; the input rows of the tile are staged in shared memory
-// (one coalesced pass), then thread (tx, ty) computes column tx, rows
-// ty*RO .. ty*RO + RO - 1 of the tile from a register window.
-constexpr int CT_X = 32, CT_Y = 8;
-
-// afb1d along the rows axis: in [B][2][H][W] -> out [B][4][Ho][W]; thread =
-// column j and RO consecutive output rows, its 2 RO + L - 2 input rows held
-// in registers (read through L1: the windows of neighbouring row groups
-// overlap).
-template <int L, int RO>
-__global__ void __launch_bounds__(128) afb_cols_t(const float *__restrict__ in,
-                                                  float *__restrict__ out, int B, int H, int W,
-                                                  int Ho, int padl,
-                                                  const __grid_constant__ TapPair t) {
-  const int ncolb = (W + blockDim.x - 1) / blockDim.x;
-  const int ngrp = (Ho + RO - 1) / RO;
-  const long long blk = blockIdx.x;
-  const int j = (int)(blk % ncolb) * blockDim.x + threadIdx.x;
-  const long long rest = blk / ncolb;
-  const long long bc = rest / ngrp;
-  const int i0 = (int)(rest - bc * ngrp) * RO;
-  if (j >= W) return;
-  const float *col = in + bc * H * W + j;
-  constexpr int NV = 2 * RO + L - 2;
-  float v[NV];
-  const int r0 = 2 * i0 - padl;
-  if (r0 >= 0 && r0 + NV <= H) {
+// Synthesis of 2 M consecutive outputs, the first at an even place t = 2 m0: with
+// tt = t + L - 2, the taps k = tt & 1, tt & 1 + 2, ... meet h = (tt - k) / 2,
+// which is m + L/2 - 1 - q for tap 2 q of output 2 m and for tap 2 q + 1 of
+// output 2 m + 1 alike.  win(i) = the (lo, hi) samples at h = m0 + i, zero
+// outside the band (a term of value zero leaves the sum, which starts at +0, as
+// it is).
+template <int L, int M, class Win>
+__device__ __forceinline__ void synthesise(const ulonglong2 *taps, f32x2 nz, Win win,
+                                           f32x2 (&acc)[2 * M]) {
+  constexpr int NW = L / 2 + M - 1;
+  f32x2 lo[NW], hi[NW];
 #pragma unroll
-    for (int q = 0; q < NV; q++) v[q] = col[(long long)(r0 + q) * W];
-  } else {
+  for (int i = 0; i < M - 1; i++) win(NW - 1 - i, lo[NW - 1 - i], hi[NW - 1 - i]);
 #pragma unroll
-    for (int q = 0; q < NV; q++) {
-      const int rr = r0 + q;
-      v[q] = col[(long long)(rr >= 0 && rr < H ? rr : reflect(rr, H)) * W];
+  for (int r = 0; r < 2 * M; r++) acc[r] = 0ull;
+#pragma unroll
+  for (int q = 0; q < L / 2; q++) {
+    const int i0 = L / 2 - 1 - q;
+    win(i0, lo[i0], hi[i0]);
+#pragma unroll
+    for (int p = 0; p < 2; p++) {
+      const ulonglong2 c = taps[2 * q + p];
+#pragma unroll
+      for (int m = 0; m < M; m++)
+        acc[2 * m + p] = add2(acc[2 * m + p],
+                              add2(mul2(c.x, lo[i0 + m], nz), mul2(c.y, hi[i0 + m], nz)));
     }
+  }
+}
+
+// A warp's RO consecutive outputs per lane of NC rows, written through its shared
+// buffer (32 NC RO floats) so that the stores run along the rows.  e0 = the warp's
+// first group, ngrp groups per row; store(r, j, value) with r the block's pair of
+// rows, j the column, value(c) the output of the c-th of its rows.
+template <int RO, int NC, class Value, class Store>
+__device__ __forceinline__ void store_rows(float *buf, Value value, int e0, int ngrp, int egrp,
+                                           Store store) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < NC; c++)
+#pragma unroll
+    for (int o = 0; o < RO; o += 4)
+      *reinterpret_cast<float4 *>(buf + (c * 32 + lane) * RO + o) =
+          make_float4(value(c, o), value(c, o + 1), value(c, o + 2), value(c, o + 3));
+  __syncwarp();
+  int r = e0 / ngrp, g = e0 - r * ngrp + lane / RO;
+#pragma unroll
+  for (int i = 0; i < RO; i++, g += 32 / RO) {
+    if (e0 + lane / RO + i * (32 / RO) >= egrp) break;
+    while (g >= ngrp) g -= ngrp, r++;
+    store(r, g * RO + lane % RO, [=](int c) { return buf[(c * RO + i) * 32 + lane]; });
+  }
+}
+
+constexpr int FB_PAIRS = 16;  // pairs of rows per block, at most
+
+// Shared memory places of a row of n staged samples, one skipped after every g
+// (an even count: the buffers behind are read in 16-byte pieces).
+__host__ __device__ inline int fw_pad(int n, int g) { return (n + n / g + 2) & ~1; }
+
+// afb1d along the last axis, two rows at a time: RB pairs of rows (of all the
+// chunk's rows in a line) per block are staged in shared memory as float2 (row
+// 2 i, row 2 i + 1) with the symmetric extension applied, one place skipped after
+// every 2 RO so that lanes RO outputs apart meet different banks.
+template <int L, int RO>
+__global__ void __launch_bounds__(320) afb_rows_t(const float *__restrict__ x, long long sz,
+                                                  int sx, float *__restrict__ out, int B, int H,
+                                                  int W, int Wo, int padl, int RB,
+                                                  const __grid_constant__ TapPair t) {
+  extern __shared__ __align__(16) f32x2 frow[];
+  __shared__ ulonglong2 taps[L];
+  const f32x2 nz = stage_taps<L>(taps, t);
+  const int ngrp = (Wo + RO - 1) / RO;
+  const int SW = 2 * RO * ngrp + L - 2, SP = fw_pad(SW, 2 * RO);
+  float *buf = reinterpret_cast<float *>(frow + RB * SP) + (threadIdx.x / 32) * 128 * RO;
+  const long long nrows = (long long)B * H, row0 = 2LL * blockIdx.x * RB;
+  const int np = (int)min((long long)RB, (nrows - row0 + 1) / 2);
+  const long long band = (long long)H * Wo;
+  __shared__ float *orow[2 * FB_PAIRS];  // the rows' low bands, null past the last row
+  if (threadIdx.x < 2 * np) {
+    const long long row = row0 + threadIdx.x;
+    orow[threadIdx.x] = row < nrows ? out + row / H * 2 * band + row % H * Wo : nullptr;
+  }
+  for (int r = 0; r < np; r++) {
+    const long long ra = row0 + 2 * r, rb = min(ra + 1, nrows - 1);
+    const float *xa = x + ra / H * sz + ra % H * sx, *xb = x + rb / H * sz + rb % H * sx;
+    f32x2 *sr = frow + r * SP;
+#pragma unroll 4
+    for (int u = threadIdx.x; u < SW; u += blockDim.x) {
+      int m = u - padl;
+      if ((unsigned)m >= (unsigned)W) m = reflect(m, W);
+      sr[u + u / (2 * RO)] = pack2(xa[m], xb[m]);
+    }
+  }
+  __syncthreads();
+  const int egrp = np * ngrp;
+  for (int e0 = threadIdx.x & ~31; e0 < egrp; e0 += blockDim.x) {
+    const int e = min(e0 + (int)(threadIdx.x & 31), egrp - 1);
+    const int r = e / ngrp, g = e - r * ngrp;
+    const f32x2 *p = frow + r * SP + g * (2 * RO + 1);
+    f32x2 lo[RO], hi[RO];
+    analyse<L, RO>(taps, nz, [p](int q) { return p[q + q / (2 * RO)]; }, lo, hi);
+    // low and high band of the first row, of the second
+    store_rows<RO, 4>(
+        buf,
+        [&](int c, int o) {
+          const float2 w = unpack2(c & 1 ? hi[o] : lo[o]);
+          return c & 2 ? w.y : w.x;
+        },
+        e0, ngrp, egrp, [&](int rr, int j, auto val) {
+          if (j >= Wo) return;
+          float *oa = orow[2 * rr], *ob = orow[2 * rr + 1];
+          oa[j] = val(0);
+          oa[band + j] = val(1);
+          if (ob) ob[j] = val(2), ob[band + j] = val(3);
+        });
+  }
+}
+
+// Column kernels: a warp takes 64 columns (a lane's two 32 apart in the halves of
+// the packed values) and 8 warps adjacent runs of outputs, whose overlapping
+// inputs meet in L1.
+
+// afb1d along the rows axis: in [B][2][H][W] -> out [B][4][Ho][W].
+template <int L, int RO>
+__global__ void __launch_bounds__(256, 2) afb_cols_t(const float *__restrict__ in,
+                                                     float *__restrict__ out, int B, int H, int W,
+                                                     int Ho, int padl,
+                                                     const __grid_constant__ TapPair t) {
+  __shared__ ulonglong2 taps[L];
+  const f32x2 nz = stage_taps<L>(taps, t);
+  __syncthreads();
+  const int ncolb = (W + 63) / 64;
+  const int ngrp = (Ho + 8 * RO - 1) / (8 * RO);
+  const unsigned blk = blockIdx.x;
+  const int j = (int)(blk % ncolb) * 64 + threadIdx.x % 32;
+  const unsigned rest = blk / ncolb;
+  const long long bc = rest / ngrp;
+  const int i0 = ((int)(rest % ngrp) * 8 + threadIdx.x / 32) * RO;
+  if (i0 >= Ho) return;
+  const float *ca = in + bc * H * W + min(j, W - 1), *cb = in + bc * H * W + min(j + 32, W - 1);
+  const int r0 = 2 * i0 - padl;
+  f32x2 lo[RO], hi[RO];
+  if (r0 >= 0 && r0 + 2 * RO + L - 2 <= H) {
+    ca += (long long)r0 * W;
+    cb += (long long)r0 * W;
+    analyse<L, RO>(taps, nz, [=](int q) { return pack2(ca[q * W], cb[q * W]); }, lo, hi);
+  } else {
+    analyse<L, RO>(taps, nz, [=](int q) {
+      int rr = r0 + q;
+      if ((unsigned)rr >= (unsigned)H) rr = reflect(rr, H);
+      return pack2(ca[(long long)rr * W], cb[(long long)rr * W]);
+    }, lo, hi);
   }
   const long long b = bc / 2, c = bc % 2;
-  float *o0 = out + ((b * 4 + 2 * c) * Ho) * (long long)W + j;
+  float *o0 = out + ((b * 4 + 2 * c) * Ho + i0) * (long long)W + j;
   float *o1 = o0 + (long long)Ho * W;
-  float lo[RO], hi[RO];
-#pragma unroll
-  for (int r = 0; r < RO; r++) {
-    lo[r] = __fmul_rn(t.a[0], v[2 * r]);
-    hi[r] = __fmul_rn(t.b[0], v[2 * r]);
-  }
-#pragma unroll
-  for (int k = 1; k < L; k++) {
-    const float ak = t.a[k], bk = t.b[k];
-#pragma unroll
-    for (int r = 0; r < RO; r++) {
-      lo[r] = __fadd_rn(lo[r], __fmul_rn(ak, v[2 * r + k]));
-      hi[r] = __fadd_rn(hi[r], __fmul_rn(bk, v[2 * r + k]));
-    }
-  }
+  const bool oka = j < W, okb = j + 32 < W;
 #pragma unroll
   for (int r = 0; r < RO; r++)
     if (i0 + r < Ho) {
-      o0[(long long)(i0 + r) * W] = lo[r];
-      o1[(long long)(i0 + r) * W] = hi[r];
+      const float2 l = unpack2(lo[r]), h = unpack2(hi[r]);
+      if (oka) o0[r * W] = l.x, o1[r * W] = h.x;
+      if (okb) o0[r * W + 32] = l.y, o1[r * W + 32] = h.y;
     }
 }
 
-// One synthesis output: acc over k of the reference's parity (k = tt & 1,
-// tt & 1 + 2, ...), h = (tt - k)/2 skipped outside [0, Hi).  Windows lo/hi
-// hold h = hb + idx; RO consecutive outputs with tt0 even (L even), so
-// h = hb + L/2 + (r - k)/2.
-template <int L, int RO, bool CHECK>
-__device__ __forceinline__ void synth_outputs(const float (&lo)[L / 2 + RO / 2],
-                                              const float (&hi)[L / 2 + RO / 2], int hb, int Hi,
-                                              const TapPair &t, float (&acc)[RO]) {
-#pragma unroll
-  for (int r = 0; r < RO; r++) acc[r] = 0.f;
-#pragma unroll
-  for (int k = 0; k < L; k++) {
-    const float ak = t.a[k], bk = t.b[k];
-#pragma unroll
-    for (int r = k & 1; r < RO; r += 2) {
-      const int idx = (r - k) / 2 + L / 2;  // h - hb
-      if (CHECK) {
-        const int h = hb + idx;
-        if (h < 0 || h >= Hi) continue;
-      }
-      const float vv = __fadd_rn(__fmul_rn(ak, lo[idx]), __fmul_rn(bk, hi[idx]));
-      acc[r] = __fadd_rn(acc[r], vv);
-    }
-  }
-}
-
-// sfb1d along the rows axis (see sfb_cols): tile rows t0.. (t0 a multiple
-// of 8 * RO, so every thread's first output row is even).
-template <int L, int RO>
-__global__ void __launch_bounds__(CT_X *CT_Y) sfb_cols_t(const float *__restrict__ y,
-                                                         long long bstride, int Hi, int Wb, int W,
-                                                         float *__restrict__ out, int B, int Ho,
-                                                         const __grid_constant__ TapPair t) {
-  static_assert(L % 2 == 0 && RO % 2 == 0, "even filter length and output block");
-  constexpr int TR = CT_Y * RO;
-  constexpr int NW = L / 2 + RO / 2;       // window per thread
-  constexpr int NT = TR / 2 + L / 2;       // window per tile
-  __shared__ float tlo[NT][CT_X], thi[NT][CT_X];
-  const int ncolb = (W + CT_X - 1) / CT_X;
-  const int ngrp = (Ho + TR - 1) / TR;
-  const long long blk = blockIdx.x;
-  const int cb = (int)(blk % ncolb);
-  const long long rest = blk / ncolb;
+// sfb1d along the rows axis (see sfb_cols).
+template <int L, int M>
+__global__ void __launch_bounds__(256, 2) sfb_cols_t(const float *__restrict__ y,
+                                                     long long bstride, int Hi, int Wb, int W,
+                                                     float *__restrict__ out, int B, int Ho,
+                                                     const __grid_constant__ TapPair t) {
+  static_assert(L % 2 == 0, "even filter length");
+  __shared__ ulonglong2 taps[L];
+  const f32x2 nz = stage_taps<L>(taps, t);
+  __syncthreads();
+  const int ncolb = (W + 63) / 64;
+  const int ngrp = (Ho + 16 * M - 1) / (16 * M);
+  const unsigned blk = blockIdx.x;
+  const int j = (int)(blk % ncolb) * 64 + threadIdx.x % 32;
+  const unsigned rest = blk / ncolb;
   const long long bc = rest / ngrp;
-  const int t0 = (int)(rest - bc * ngrp) * TR;
-  const int tx = threadIdx.x % CT_X, ty = threadIdx.x / CT_X;
-  const int j = cb * CT_X + tx;
+  const int t0 = ((int)(rest % ngrp) * 8 + threadIdx.x / 32) * 2 * M;
+  if (t0 >= Ho) return;
   const int b = (int)(bc / 2), c = (int)(bc % 2);
   const long long plane = (long long)Hi * Wb;
-  const float *base = y + b * bstride;
-  const float *lop = base + (c == 0 ? 0 : 2) * plane + j;  // LL or band1 (HL)
-  const float *hip = base + (c == 0 ? 1 : 3) * plane + j;  // band0 (LH) or band2 (HH)
-  const int hbt = (t0 + L - 2) / 2 - L / 2;  // h of tile window index 0
-  for (int q = ty; q < NT; q += CT_Y) {
-    const int h = hbt + q;
-    const bool ok = j < W && h >= 0 && h < Hi;
-    tlo[q][tx] = ok ? lop[(long long)h * Wb] : 0.f;
-    thi[q][tx] = ok ? hip[(long long)h * Wb] : 0.f;
+  // channel 0 = LL and band 0 (LH), channel 1 = band 1 (HL) and band 2 (HH)
+  const float *la = y + b * bstride + (c == 0 ? 0 : 2) * plane;
+  const float *lb = la + min(j + 32, W - 1);
+  la += min(j, W - 1);
+  const int h0 = t0 / 2;
+  f32x2 acc[2 * M];
+  if (h0 + L / 2 + M - 1 <= Hi) {
+    la += (long long)h0 * Wb;
+    lb += (long long)h0 * Wb;
+    const float *ha = la + plane, *hb = lb + plane;
+    synthesise<L, M>(taps, nz, [=](int i, f32x2 &lo, f32x2 &hi) {
+      lo = pack2(la[i * Wb], lb[i * Wb]);
+      hi = pack2(ha[i * Wb], hb[i * Wb]);
+    }, acc);
+  } else {
+    synthesise<L, M>(taps, nz, [=](int i, f32x2 &lo, f32x2 &hi) {
+      const long long o = (long long)(h0 + i) * Wb;
+      const bool ok = h0 + i < Hi;
+      lo = ok ? pack2(la[o], lb[o]) : 0ull;
+      hi = ok ? pack2(la[plane + o], lb[plane + o]) : 0ull;
+    }, acc);
   }
-  __syncthreads();
-  if (j >= W) return;
-  const int hb = hbt + ty * (RO / 2);
-  float lo[NW], hi[NW];
+  float *o0 = out + (bc * Ho + t0) * W + j;
+  const bool oka = j < W, okb = j + 32 < W;
 #pragma unroll
-  for (int q = 0; q < NW; q++) {
-    lo[q] = tlo[ty * (RO / 2) + q][tx];
-    hi[q] = thi[ty * (RO / 2) + q][tx];
-  }
-  float acc[RO];
-  if (hb >= 0 && hb + NW <= Hi)
-    synth_outputs<L, RO, false>(lo, hi, hb, Hi, t, acc);
-  else
-    synth_outputs<L, RO, true>(lo, hi, hb, Hi, t, acc);
-  const int tt0 = t0 + ty * RO;
-#pragma unroll
-  for (int r = 0; r < RO; r++)
-    if (tt0 + r < Ho) out[(bc * Ho + tt0 + r) * W + j] = acc[r];
+  for (int r = 0; r < 2 * M; r++)
+    if (t0 + r < Ho) {
+      const float2 v = unpack2(acc[r]);
+      if (oka) o0[r * W] = v.x;
+      if (okb) o0[r * W + 32] = v.y;
+    }
 }
 
-// sfb1d along the last axis (see sfb_rows): thread = RO consecutive outputs
-// w0.. of one row (w0 a multiple of RO), windows read through L1.
-template <int L, int RO>
-__global__ void __launch_bounds__(128) sfb_rows_t(const float *__restrict__ in, int H, int Wi,
+// sfb1d along the last axis (see sfb_rows), two rows at a time: RB pairs of rows
+// per block staged as float4 (low and high band of the first row and the second:
+// the packed low, the packed high), one place skipped after every M.
+template <int L, int M>
+__global__ void __launch_bounds__(320) sfb_rows_t(const float *__restrict__ in, int H, int Wi,
                                                   float *__restrict__ dst, long long dsz, int dsx,
-                                                  int Hd, int Wd, int B,
+                                                  int Hd, int Wd, int B, int RB,
                                                   const __grid_constant__ TapPair t) {
-  const int ngrp = (Wd + RO - 1) / RO;
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= (long long)B * Hd * ngrp) return;
-  const int w0 = (int)(g % ngrp) * RO;
-  const long long rowi = g / ngrp;
-  const int h = (int)(rowi % Hd);
-  const int b = (int)(rowi / Hd);
-  const float *lop = in + (((long long)b * 2) * H + h) * Wi;
-  const float *hip = lop + (long long)H * Wi;
-  constexpr int NW = L / 2 + RO / 2;
-  const int hb = (w0 + L - 2) / 2 - L / 2;
-  float lo[NW], hi[NW];
-#pragma unroll
-  for (int q = 0; q < NW; q++) {
-    const int qq = hb + q;
-    const bool ok = qq >= 0 && qq < Wi;
-    lo[q] = ok ? lop[qq] : 0.f;
-    hi[q] = ok ? hip[qq] : 0.f;
+  extern __shared__ __align__(16) f32x2 frow[];
+  __shared__ ulonglong2 taps[L];
+  const f32x2 nz = stage_taps<L>(taps, t);
+  const int ngrp = (Wd + 2 * M - 1) / (2 * M);
+  const int SW = M * ngrp + L / 2 - 1, SP = fw_pad(SW, M);
+  ulonglong2 *srow = reinterpret_cast<ulonglong2 *>(frow);
+  float *buf = reinterpret_cast<float *>(srow + RB * SP) + (threadIdx.x / 32) * 128 * M;
+  const long long nrows = (long long)B * Hd, row0 = 2LL * blockIdx.x * RB;
+  const int np = (int)min((long long)RB, (nrows - row0 + 1) / 2);
+  const long long band = (long long)H * Wi;
+  __shared__ float *orow[2 * FB_PAIRS];  // output rows, null past the last
+  if (threadIdx.x < 2 * np) {
+    const long long row = row0 + threadIdx.x;
+    orow[threadIdx.x] = row < nrows ? dst + row / Hd * dsz + row % Hd * dsx : nullptr;
   }
-  float acc[RO];
-  if (hb >= 0 && hb + NW <= Wi)
-    synth_outputs<L, RO, false>(lo, hi, hb, Wi, t, acc);
-  else
-    synth_outputs<L, RO, true>(lo, hi, hb, Wi, t, acc);
-  float *d = dst + b * dsz + (long long)h * dsx;
-#pragma unroll
-  for (int r = 0; r < RO; r++)
-    if (w0 + r < Wd) d[w0 + r] = acc[r];
+  for (int r = 0; r < np; r++) {
+    const long long ra = row0 + 2 * r, rb = min(ra + 1, nrows - 1);
+    const float *la = in + (ra / Hd * 2 * H + ra % Hd) * Wi;
+    const float *lb = in + (rb / Hd * 2 * H + rb % Hd) * Wi;
+    ulonglong2 *sr = srow + r * SP;
+#pragma unroll 4
+    for (int u = threadIdx.x; u < SW; u += blockDim.x) {
+      ulonglong2 w = make_ulonglong2(0ull, 0ull);
+      if (u < Wi) {
+        w.x = pack2(la[u], lb[u]);
+        w.y = pack2(la[band + u], lb[band + u]);
+      }
+      sr[u + u / M] = w;
+    }
+  }
+  __syncthreads();
+  const int egrp = np * ngrp;
+  for (int e0 = threadIdx.x & ~31; e0 < egrp; e0 += blockDim.x) {
+    const int e = min(e0 + (int)(threadIdx.x & 31), egrp - 1);
+    const int r = e / ngrp, g = e - r * ngrp;
+    const ulonglong2 *p = srow + r * SP + g * (M + 1);
+    f32x2 acc[2 * M];
+    synthesise<L, M>(taps, nz, [p](int i, f32x2 &lo, f32x2 &hi) {
+      const ulonglong2 w = p[i + i / M];
+      lo = w.x;
+      hi = w.y;
+    }, acc);
+    store_rows<2 * M, 2>(
+        buf,
+        [&](int c, int o) {
+          const float2 w = unpack2(acc[o]);
+          return c ? w.y : w.x;
+        },
+        e0, ngrp, egrp, [&](int rr, int j, auto val) {
+          if (j >= Wd) return;
+          float *oa = orow[2 * rr], *ob = orow[2 * rr + 1];
+          oa[j] = val(0);
+          if (ob) ob[j] = val(1);
+        });
+  }
 }
 
 // [B][R][C] <-> [B][C][R] (32x32 tiles)
@@ -487,7 +591,8 @@ __global__ void damp_kernel(float2 *__restrict__ spec, const float *__restrict__
 
 // Damping by the low Fourier modes, in place on band [B][H][W] (slice
 // stride bstride): a block takes 32 adjacent columns (threadIdx.x) of one
-// slice, 8 row phases (threadIdx.y).  cs[k * H + q] = (cos, sin)(2 pi k q / H)
+// slice, 8 row phases (threadIdx.y).  cs[q * V1 + k] = (cos, sin)(2 pi k q / H)
+// (read 16 bytes at a time)
 // and gw[k] = g_k / H (k = 0) or 2 g_k / H (k >= 1, the mode and its mirror
 // H - k).  Pass 1 sums A_k = sum_q x_q cos, S_k = sum_q x_q sin per column;
 // pass 2 writes x_q - sum_k gw_k (A_k cos + S_k sin).
@@ -496,7 +601,7 @@ constexpr int DM_R = 8;
 template <int V1>
 __global__ void __launch_bounds__(32 * DM_R)
     damp_modes(float *__restrict__ band, long long bstride, int H, int W,
-               const float2 *__restrict__ cs, const float *__restrict__ gw) {
+               const float4 *__restrict__ cs, const float *__restrict__ gw) {
   __shared__ float red[DM_R][V1][32];
   const int w = blockIdx.x * 32 + threadIdx.x, r = threadIdx.y;
   float *col = band + (long long)blockIdx.y * bstride + w;
@@ -505,13 +610,16 @@ __global__ void __launch_bounds__(32 * DM_R)
 #pragma unroll
   for (int k = 0; k < V1; k++) A[k] = S[k] = 0.f;
   if (on)
+#pragma unroll 4
     for (int q = r; q < H; q += DM_R) {
       const float x = col[(long long)q * W];
 #pragma unroll
-      for (int k = 0; k < V1; k++) {
-        const float2 t = __ldg(cs + k * H + q);
+      for (int k = 0; k < V1; k += 2) {
+        const float4 t = __ldg(cs + (q * V1 + k) / 2);
         A[k] = fmaf(x, t.x, A[k]);
         S[k] = fmaf(x, t.y, S[k]);
+        A[k + 1] = fmaf(x, t.z, A[k + 1]);
+        S[k + 1] = fmaf(x, t.w, S[k + 1]);
       }
     }
   // the 8 row phases' partial sums, cosine then sine terms through one buffer
@@ -537,12 +645,14 @@ __global__ void __launch_bounds__(32 * DM_R)
     S[k] = b * __ldg(gw + k);
   }
   if (!on) return;
+#pragma unroll 4
   for (int q = r; q < H; q += DM_R) {
     float lp = 0.f;
 #pragma unroll
-    for (int k = 0; k < V1; k++) {
-      const float2 t = __ldg(cs + k * H + q);
+    for (int k = 0; k < V1; k += 2) {
+      const float4 t = __ldg(cs + (q * V1 + k) / 2);
       lp = fmaf(A[k], t.x, fmaf(S[k], t.y, lp));
+      lp = fmaf(A[k + 1], t.z, fmaf(S[k + 1], t.w, lp));
     }
     col[(long long)q * W] -= lp;
   }
@@ -561,7 +671,7 @@ struct tcb_stripe_fw {
   std::vector<float *> damp;  // per level damping factors (with 1/H)
   std::vector<cufftHandle> r2c, c2r;
   std::vector<int> modes;     // per level: modes of the direct damping (0 = cuFFT)
-  std::vector<float2 *> mcs;  // per level [modes][H] (cos, sin)(2 pi k q / H)
+  std::vector<float4 *> mcs;  // per level [H][modes] (cos, sin)(2 pi k q / H)
   std::vector<float *> mgw;   // per level [modes] weights
   float *tmp = nullptr;    // [nz][2][H][W] scratch
   float *bt = nullptr;     // transposed band scratch
@@ -572,40 +682,72 @@ struct tcb_stripe_fw {
 };
 
 namespace {
-constexpr int FB_RO = 4;  // outputs per thread of the column / synthesis kernels
+// outputs per thread: of the analysis along the rows, along the columns, and half
+// of the synthesis'
+constexpr int FB_RO = 4, FB_CO = 8, FB_M = 4;
+// wide rows' shared memory (one value for every call: threads may launch at once)
+constexpr int FB_MAX_SMEM = 220 * 1024;
+
+// Pairs of rows and threads per block of a row kernel: `groups` threads' turns and
+// `bytes` of shared memory per pair.  The split that leaves the fewest lanes idle
+// in the last turn, the smaller block where they are alike.
+void rows_split(int groups, size_t bytes, int &RB, int &T) {
+  double best = 0;
+  for (int rb = 1; rb <= FB_PAIRS && (rb == 1 || rb * bytes <= 40960); rb++)
+    for (int th = 128; th <= 320; th += 32) {
+      const int turns = (rb * groups + th - 1) / th;
+      const double use = (double)rb * groups / ((double)turns * th);
+      if (use > best + 0.02) best = use, RB = rb, T = th;
+    }
+}
 
 template <int L>
 void launch_afb_rows(const tcb_stripe_fw *h, const float *x, long long xsz, int xsx, int B,
                      int Hk, int Wk, int Wo, int padl, cudaStream_t s) {
-  const int SW = 2 * ((Wo + 3) / 4 * 4) + L - 2;  // windows of the last 4-output group
-  const int RB = std::max(1, std::min(16, 1024 / Wo));
-  const long long nb = ((long long)B * Hk + RB - 1) / RB;
-  afb_rows_t<L><<<(unsigned)nb, 256, (size_t)RB * SW * sizeof(float), s>>>(
-      x, xsz, xsx, h->tmp, B, Hk, Wk, Wo, padl, RB, SW, h->ana);
+  const int ngrp = (Wo + FB_RO - 1) / FB_RO;
+  const size_t bytes = (size_t)fw_pad(2 * FB_RO * ngrp + L - 2, 2 * FB_RO) * sizeof(f32x2);
+  int RB, T;
+  rows_split(ngrp, bytes, RB, T);
+  const size_t smem = RB * bytes + (size_t)T * 4 * FB_RO * sizeof(float);
+  if (smem > 40960)
+    cudaFuncSetAttribute(afb_rows_t<L, FB_RO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         FB_MAX_SMEM);
+  const long long nb = ((long long)B * Hk + 2 * RB - 1) / (2 * RB);
+  afb_rows_t<L, FB_RO><<<(unsigned)nb, T, smem, s>>>(x, xsz, xsx, h->tmp, B, Hk, Wk, Wo, padl, RB,
+                                                     h->ana);
 }
 
 template <int L>
 void launch_afb_cols(const tcb_stripe_fw *h, float *out, int B, int Hk, int Wo, int Ho, int padl,
                      cudaStream_t s) {
-  const long long nb = (long long)ceil_div(Wo, 128) * (2LL * B) * ((Ho + FB_RO - 1) / FB_RO);
-  afb_cols_t<L, FB_RO><<<(unsigned)nb, 128, 0, s>>>(h->tmp, out, B, Hk, Wo, Ho, padl, h->ana);
+  const long long nb = (long long)ceil_div(Wo, 64) * (2LL * B) *
+                       ((Ho + 8 * FB_CO - 1) / (8 * FB_CO));
+  afb_cols_t<L, FB_CO><<<(unsigned)nb, 256, 0, s>>>(h->tmp, out, B, Hk, Wo, Ho, padl, h->ana);
 }
 
 template <int L>
 void launch_sfb_cols(const tcb_stripe_fw *h, const float *y, int Hi, int Wi, int B, int Hc,
                      cudaStream_t s) {
-  const long long nb = (long long)ceil_div(Wi, CT_X) * (2LL * B) *
-                       ((Hc + CT_Y * FB_RO - 1) / (CT_Y * FB_RO));
-  sfb_cols_t<L, FB_RO><<<(unsigned)nb, CT_X * CT_Y, 0, s>>>(y, 4LL * Hi * Wi, Hi, Wi, Wi,
-                                                            h->tmp, B, Hc, h->syn);
+  const long long nb = (long long)ceil_div(Wi, 64) * (2LL * B) *
+                       ((Hc + 16 * FB_M - 1) / (16 * FB_M));
+  sfb_cols_t<L, FB_M><<<(unsigned)nb, 256, 0, s>>>(y, 4LL * Hi * Wi, Hi, Wi, Wi, h->tmp, B, Hc,
+                                                   h->syn);
 }
 
 template <int L>
 void launch_sfb_rows(const tcb_stripe_fw *h, int Hc, int Wi, float *dst, long long dsz, int Wd,
                      int Hrows, int B, cudaStream_t s) {
-  const long long thr = (long long)B * Hrows * ((Wd + FB_RO - 1) / FB_RO);
-  sfb_rows_t<L, FB_RO><<<(unsigned)ceil_div(thr, 128), 128, 0, s>>>(h->tmp, Hc, Wi, dst, dsz, Wd,
-                                                                    Hrows, Wd, B, h->syn);
+  const int ngrp = (Wd + 2 * FB_M - 1) / (2 * FB_M);
+  const size_t bytes = (size_t)fw_pad(FB_M * ngrp + L / 2 - 1, FB_M) * sizeof(ulonglong2);
+  int RB, T;
+  rows_split(ngrp, bytes, RB, T);
+  const size_t smem = RB * bytes + (size_t)T * 4 * FB_M * sizeof(float);
+  if (smem > 40960)
+    cudaFuncSetAttribute(sfb_rows_t<L, FB_M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         FB_MAX_SMEM);
+  const long long nb = ((long long)B * Hrows + 2 * RB - 1) / (2 * RB);
+  sfb_rows_t<L, FB_M><<<(unsigned)nb, T, smem, s>>>(h->tmp, Hc, Wi, dst, dsz, Wd, Hrows, Wd, B, RB,
+                                                    h->syn);
 }
 
 bool blocked_length(int L) { return L == 2 || L == 10 || L == 32; }
@@ -673,11 +815,10 @@ extern "C" int tcb_stripe_fw_create(tcb_stripe_fw **out, size_t nproj, size_t nz
     t.g1[k] = (float)rec_hi[k];
   }
   for (int k = 0; k < L; k++) {
-    h->ana.a[k] = t.h0[k];
-    h->ana.b[k] = t.h1[k];
-    h->syn.a[k] = t.g0[k];
-    h->syn.b[k] = t.g1[k];
+    h->ana.c[k] = make_float4(t.h0[k], t.h0[k], t.h1[k], t.h1[k]);
+    h->syn.c[k] = make_float4(t.g0[k], t.g0[k], t.g1[k], t.g1[k]);
   }
+  h->ana.nz = h->syn.nz = make_float2(-0.f, -0.f);
   if (cudaMalloc(&h->taps, sizeof(Taps)) != cudaSuccess)
     return fail(TCB_ERR_OUT_OF_MEMORY, "cudaMalloc failed");
   if (cudaMemcpy(h->taps, &t, sizeof(Taps), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -734,7 +875,7 @@ extern "C" int tcb_stripe_fw_create(tcb_stripe_fw **out, size_t nproj, size_t nz
         for (int q = 0; q < Ho; q++) {
           // 2 pi k q / H reduced exactly: (k q mod H) / H
           const double a = 2.0 * M_PI * (double)(((long long)k * q) % Ho) / (double)Ho;
-          tab[(size_t)k * Ho + q] = make_float2((float)std::cos(a), (float)std::sin(a));
+          tab[(size_t)q * V1 + k] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
         const double v = (Ho % 2) ? (double)k : k + 0.5;
         const double g = std::exp(-v * v / (2.0 * (double)sigma * sigma)) / Ho;
@@ -756,7 +897,7 @@ extern "C" int tcb_stripe_fw_create(tcb_stripe_fw **out, size_t nproj, size_t nz
       }
     }
     h->modes.push_back(V1);
-    h->mcs.push_back(mc);
+    h->mcs.push_back(reinterpret_cast<float4 *>(mc));
     h->mgw.push_back(mg);
     maxband = std::max(maxband, (size_t)nz * Ho * Wo);
     maxtmp = std::max(maxtmp, (size_t)nz * 2 * h->H[k] * Wo);          // afb rows output
