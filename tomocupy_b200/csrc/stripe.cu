@@ -215,8 +215,9 @@ __global__ void sfb_rows(const float *__restrict__ in, int H, int Wi, float *__r
 // These instructions (two cycles of the FP32 pipe each) are the bound: 0.13 ms per
 // pass over the 7 levels of 16 slices of 1500 x 2048 at 32 taps.  Measured there,
 // one output at a time and packed: analysis rows 0.45 and 0.44 ms, columns 0.40
-// and 0.36, synthesis columns 0.51 and 0.36, rows 0.41 and 0.40; what is left is
-// the staging's latency (rows) and the few warps 127 registers leave (columns).
+// and 0.36, synthesis columns 0.51 and 0.33, rows 0.41 and 0.40; what is left is
+// the staging's latency (rows) and the few warps 127 registers leave (columns of the
+// analysis; the synthesis gains from three blocks per SM at 80: 0.36 with two).
 struct TapPair {
   float4 c[MAXL];  // (a, a, b, b) of tap k
   float2 nz;       // -0, -0
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(256, 2) afb_cols_t(const float *__restrict__ i
 
 // sfb1d along the rows axis (see sfb_cols).
 template <int L, int M>
-__global__ void __launch_bounds__(256, 2) sfb_cols_t(const float *__restrict__ y,
+__global__ void __launch_bounds__(256, 3) sfb_cols_t(const float *__restrict__ y,
                                                      long long bstride, int Hi, int Wb, int W,
                                                      float *__restrict__ out, int B, int Ho,
                                                      const __grid_constant__ TapPair t) {
