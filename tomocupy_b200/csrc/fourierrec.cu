@@ -1093,7 +1093,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
 }
 
 // Persistent and warp-specialised: CTA b takes the work items (tile, pair
-// group) b, b + G, ... of tile_order (raster order by rounds of G, balanced).  The producer warp streams the
+// group) b, b + G, ... of tile_order (raster order by rounds of G, balanced).  The producer warps stream the
 // chunks of all its items through NST stages (W by bulk copies that complete
 // on the stage's mbarrier, V rows by cp.async whose lanes arrive on it once
 // their gathers have landed), prefetching the next chunk's row indices and
