@@ -18,6 +18,7 @@ usfft2d stage reads S1 in place (``cfunc_usfft2d.adj_rows``).
 """
 from __future__ import annotations
 
+import functools
 import math
 
 import numpy as np
@@ -47,9 +48,9 @@ class BackprojLamFourierParallel:
         self.cl_lamfourier = lamfourierrec.LamFourierRec(
             self.n0, self.n1, self.n2, self.ntheta, self.detw, self.deth, self.n1c,
             self.nthetac, self.dethc)
-        # filter applied along the rows of each projection (not sinograms)
-        self.cl_filter = fbp_filter.FBPFilter(self.ne, self.deth, self.nthetac, args.dtype)
-        self.wfilter = torch.as_tensor(self.cl_filter.calc_filter(args.fbp_filter),
+        # filter applied along the rows of each projection (not sinograms); center
+        # and wfilter may be changed between calls
+        self.wfilter = torch.as_tensor(fbp_filter.calc_filter(self.ne, args.fbp_filter),
                                        device=self.device)
         self.pad = self.ne // 2 - self.detw // 2
         self.t = rfftfreq32(self.ne, self.device)
@@ -62,17 +63,46 @@ class BackprojLamFourierParallel:
         # an axis a whole number of pixels from the middle: otherwise the filter's
         # Nyquist term is complex, and cuFFT's inverse real transform, which the
         # padded chain uses, takes its imaginary part in as well at some sizes.
-        self._fff = self._rows = None
-        if (fftfilter.supported(self.detw) and self.nthetac % 2 == 0 and args.dtype != "float16"
-                and float(self.center - self.detw / 2).is_integer()):
-            self._fff = fftfilter.FFTFilter(self.detw, self.deth, self.nthetac, 1, self.device)
-            self._fff.set_kernels(self.cl_filter.calc_filter(args.fbp_filter), self.ne,
-                                  self.center, 0.0)
-        else:
-            self._rows = torch.empty((self.nthetac, self.deth, self.ne), dtype=torch.float32,
-                                     device=self.device)
+        # Only the filter that the axis asks for is built here, the other one when
+        # a later call needs it (both at once: 5.0 ms of construction at 512^2 x 600,
+        # this one 3.7, cuFFT's plans for the other stages most of it).
+        self._rows = self._fff = self._fff_of = None
+        self._can_fuse = (fftfilter.supported(self.detw) and self.nthetac % 2 == 0
+                          and args.dtype != "float16")
+        self._dtype = args.dtype
+        if self._fused() is None:
+            self._padded()
         self.cl_writer = cl_writer
         self.rec_fun = self.rec_lam
+
+    @functools.cached_property
+    def cl_filter(self):
+        """The filter on padded rows (cuFFT plans of length 4 detw)."""
+        return fbp_filter.FBPFilter(self.ne, self.deth, self.nthetac, self._dtype)
+
+    def _fused(self):
+        """The fused filter for the present ``center`` and ``wfilter``, or None
+        where the padded chain has to run."""
+        if not self._can_fuse or not float(self.center - self.detw / 2).is_integer():
+            return None
+        wf = self.wfilter.detach().cpu().numpy().copy()
+        if (wf.shape != (self.ne // 2 + 1,) or wf.dtype != np.float32
+                or not np.isfinite(wf).all()):
+            return None
+        of = float(self.center), wf
+        if self._fff is None or of[0] != self._fff_of[0] or not np.array_equal(wf, self._fff_of[1]):
+            # a new object: calls in flight still read the old one's kernels
+            fff = fftfilter.FFTFilter(self.detw, self.deth, self.nthetac, 1, self.device)
+            fff.set_kernels(wf, self.ne, of[0], 0.0)
+            self._fff, self._fff_of = fff, of
+        return self._fff
+
+    def _padded(self):
+        """The padded chain's row buffer and filter."""
+        if self._rows is None:
+            self._rows = torch.empty((self.nthetac, self.deth, self.ne), dtype=torch.float32,
+                                     device=self.device)
+        return self._rows, self.cl_filter.fslv
 
     def _weights(self, nthetac):
         # backproj_lamfourier_parallel.py:270-271: (-2*pi*i * t) * (-center + sht + n2/2)
@@ -83,28 +113,22 @@ class BackprojLamFourierParallel:
         w = torch.complex(self.wfilter * torch.cos(phase), self.wfilter * torch.sin(phase))
         return torch.view_as_real(w).contiguous()
 
-    def _filter(self, chunk, w, stream):
+    def _filter(self, chunk, fff, w, stream):
         """Filtered rows of the projections ``chunk`` [<= nthetac, deth, detw] into
-        the chunk buffer, zeros for absent projections."""
+        the front of the chunk buffer: by the fused filter ``fff``, or by the padded
+        chain with the weights ``w``."""
         cnt = chunk.shape[0]
-        if self._fff is not None and chunk.dtype == torch.float32:
-            if cnt < self.nthetac:
-                rows = torch.zeros((self.nthetac, *chunk.shape[1:]), dtype=torch.float32,
-                                   device=self.device)
-                rows[:cnt] = chunk
-                chunk = rows
-            self._fff.apply(chunk.contiguous(), self._crop, "rows", stream=stream)
+        if fff is not None:
+            fff.apply(chunk.contiguous(), self._crop[:cnt], "rows", stream=stream)
             return
-        if self._rows is None:   # float32 frames expected, others given
-            self._rows = torch.empty((self.nthetac, self.deth, self.ne), dtype=torch.float32,
-                                     device=self.device)
+        rows, filt = self._padded()
         if cnt < self.nthetac:
-            self._rows.zero_()
-        prep_rows(self._rows, chunk.permute(1, 0, 2), darkflat=False, minus_log=False,
+            rows.zero_()
+        prep_rows(rows, chunk.permute(1, 0, 2), darkflat=False, minus_log=False,
                   out_zstride=self.deth * self.ne, out_pstride=self.ne, out_xoff=self.pad,
                   out_width=self.ne, edge_pad=True, stream=stream)
-        self.cl_filter.fslv.filter(self._rows, w, stream)
-        self._crop.copy_(self._rows[:, :, self.pad:self.pad + self.detw])
+        filt.filter(rows, w, stream)
+        self._crop.copy_(rows[:, :, self.pad:self.pad + self.detw])
 
     def rec_lam(self, data, stream=None):
         """data [ntheta, deth, detw] float32 (host or device) -> volume [rh, n1, n2]."""
@@ -112,7 +136,8 @@ class BackprojLamFourierParallel:
         phi = math.pi / 2 + params.lamino_angle / 180 * math.pi
         theta = torch.as_tensor(np.asarray(params.theta, dtype=np.float32), device=dev)
         nthetac, deth, detw = self.nthetac, self.deth, self.detw
-        w = self._weights(nthetac)
+        fff = self._fused() if data.dtype == torch.float32 else None
+        w = self._weights(nthetac) if fff is None else None
         # fp16 storage of the two stage arrays (fp32 arithmetic) in mixed precision
         half = args.dtype in ("mixed", "float16")  # fp16 storage of the stage arrays
         sdt = torch.float16 if half else torch.float32
@@ -132,7 +157,7 @@ class BackprojLamFourierParallel:
             chunk = data[st:end]
             if chunk.device != dev:
                 chunk = chunk.to(dev, non_blocking=True)
-            self._filter(chunk, w, stream)
+            self._filter(chunk, fff, w, stream)
             if not half and end - st == nthetac:   # straight into the stage array
                 self.cl_lamfourier.fft2d_fwd(s1[st:end], self._crop, stream)
                 continue
