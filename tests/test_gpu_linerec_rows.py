@@ -35,3 +35,23 @@ def test_rows_equal_bilinear(cuda, monkeypatch, n, nproj, nz, ncz, sz, bad):
     assert not op.timed_out()
     assert torch.equal(rows.isnan(), full.isnan())
     assert torch.equal(rows.nan_to_num(0.0), full.nan_to_num(0.0))
+
+
+def test_rows_beside_a_sum_that_overflows(cuda, monkeypatch):
+    """A slice next to one whose finite samples add up to infinity stays finite."""
+    import torch
+    from tomocupy_b200.cfunc_linerec import cfunc_linerec
+    n, nproj, nz = 64, 40, 12
+    data = torch.randn((nz, nproj, n), generator=torch.Generator(device=cuda).manual_seed(3),
+                       device=cuda)
+    data[5] = 2e37
+    th = torch.as_tensor((np.arange(nproj) * math.pi / nproj + 0.01).astype(np.float32),
+                         device=cuda)
+    op = cfunc_linerec(nproj, nz, n, nproj, nz)
+    rows, full = (torch.zeros((nz, n, n), device=cuda) for _ in range(2))
+    stream = torch.cuda.current_stream()
+    op.backprojection(rows, data, th, math.pi / 2, 0, stream)
+    monkeypatch.setenv("TCB_LINEREC_TMA", "0")
+    op.backprojection(full, data, th, math.pi / 2, 0, stream)
+    assert torch.isinf(full[5]).any() and torch.isfinite(full[[4, 6]]).all()
+    assert torch.equal(rows, full)

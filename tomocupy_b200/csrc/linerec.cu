@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(BX *BY)
 // which is what the bilinear sum of lr_interp rounds to when its other two
 // weights are zero; the sums are bit-identical to backproject_full_tma's.  The
 // other row's two samples enter there times zero, which matters only when they
-// are not finite: the sum of that row (the neighbouring slice's) is added times
-// zero at the end.
+// are not finite: where the sum of that row (the neighbouring slice's) is not, its
+// samples are looked through at the end (row_zero; a sum may also overflow).
 //
 // Z consecutive slices per thread (8, or 4 where that leaves fewer slices
 // unused) share the column arithmetic; rows go in pairs through packed FP32
@@ -426,8 +426,23 @@ __device__ __forceinline__ unsigned long long lr_lerp2(unsigned long long a, uns
   return r;
 }
 
+// What the samples of a slice's sinogram [nproj][n] that a voxel meets add when they
+// are multiplied by zero: NaN when one of them is not finite, else 0.
+__device__ __noinline__ float row_zero(const float *sino, const float *theta, int nproj, int n,
+                                       float fx, float fy) {
+  float sum = 0.f;
+  for (int p = 0; p < nproj; p++) {
+    const float u = lr_u(__cosf(theta[p]), __sinf(theta[p]), fx, fy, (float)(n / 2));
+    const int ur = (int)(u - 1e-5f);
+    if (ur < 0 || ur >= n - 1) continue;
+    const float *d = sino + (size_t)p * n + ur;
+    sum += 0.f * d[0] + 0.f * d[1];
+  }
+  return sum;
+}
+
 template <int Z>
-__global__ void __launch_bounds__(BX *BY)
+__global__ void __launch_bounds__(BX *BY, Z == 4 ? 6 : 4)
     backproject_rows_tma(float *__restrict__ f, const float *__restrict__ data,
                          const __grid_constant__ CUtensorMap map,
                          const float *__restrict__ theta, float c, int sz, int ncz, int n, int nz,
@@ -575,7 +590,13 @@ __global__ void __launch_bounds__(BX *BY)
     const float v = __fadd_rn((float)(tz + sz - nz / 2), (float)(nz / 2));
     const int vr = (int)(v - 1e-5f);
     float sum = 0.f;
-    if ((vr >= 0) & (vr < nz - 1)) sum = __fmaf_rn(0.f, (v - vr) > 0.5f ? a[s] : a[s + 2], a[s + 1]);
+    if ((vr >= 0) & (vr < nz - 1)) {
+      const int k = (v - vr) > 0.5f ? 0 : 2;  // the other row, v0 + s + k = vr or vr + 1
+      float other = k ? a[s + 2] : a[s];
+      if (!isfinite(other))
+        other = row_zero(data + (size_t)(v0 + s + k) * nproj * n, theta, nproj, n, fx, fy);
+      sum = __fmaf_rn(0.f, other, a[s + 1]);
+    }
     float *o = f + tx + (size_t)(n - ty - 1) * n + (size_t)tz * n * n;
     *o = __fmaf_rn(sum, c, *o);
   }
