@@ -68,6 +68,9 @@ __device__ __forceinline__ float fdecode(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
+// The same with every NaN last: the order that the medians take ranks in.
+__device__ __forceinline__ uint32_t med_key(float f) { return f != f ? 0xFFFFFFFFu : fkey(f); }
+
 // One CTA per column (z, x): the nproj values sorted ascending, ties in angle
 // order; srt/ids [(z * ni + x) * nproj + r].  Stable radix sort of the order bits,
 // four passes of 8 bits: warp w holds the items w*32*E + e*32 + lane (ascending in
@@ -188,11 +191,13 @@ void sort_columns(const float *tt, int nproj, int ni, int nz, float *srt, int *i
 // dependent shared-memory loads bounds it, so the places of the leaving and of
 // the entering value are searched for together and the values between them move
 // four at a time (one by one, after one search: 1.08 ms for windows of 61 and 21
-// on 16 x 720 x 1024; so 0.58).
+// on 16 x 720 x 1024; so 0.58).  The window holds order keys, not floats: a NaN
+// (a pixel with zero flat and dark) has its place too, so the window stays sorted
+// while the NaN passes and after it has left.
 __global__ void __launch_bounds__(VO_MED_T)
     vo_median_x(const float *__restrict__ in, float *__restrict__ out, int nz, int ni, int R,
                 int w) {
-  extern __shared__ float win[];  // win[j * VO_MED_T + t]
+  extern __shared__ uint32_t wkey[];  // wkey[j * VO_MED_T + t]
   const int t = threadIdx.x;
   const long long g = (long long)blockIdx.x * VO_MED_T + t;
   const int nrun = (ni + VO_RUN - 1) / VO_RUN;
@@ -201,10 +206,10 @@ __global__ void __launch_bounds__(VO_MED_T)
   const long long q = g / R;
   const int run = (int)(q % nrun), z = (int)(q / nrun);
   const int x0 = run * VO_RUN, x1 = min(ni, x0 + VO_RUN), h = w / 2;
-  auto val = [&](int x) { return in[((size_t)z * ni + reflect_idx(x, ni)) * R + r]; };
-  auto W = [&](int i) -> float & { return win[i * VO_MED_T + t]; };
+  auto val = [&](int x) { return med_key(in[((size_t)z * ni + reflect_idx(x, ni)) * R + r]); };
+  auto W = [&](int i) -> uint32_t & { return wkey[i * VO_MED_T + t]; };
   for (int j = 0; j < w; j++) {  // insertion sort of the first window
-    const float v = val(x0 - h + j);
+    const uint32_t v = val(x0 - h + j);
     int i = j;
     while (i > 0 && W(i - 1) > v) {
       W(i) = W(i - 1);
@@ -212,14 +217,14 @@ __global__ void __launch_bounds__(VO_MED_T)
     }
     W(i) = v;
   }
-  out[((size_t)z * ni + x0) * R + r] = W(h);
+  out[((size_t)z * ni + x0) * R + r] = fdecode(W(h));
   for (int x = x0 + 1; x < x1; x++) {
-    const float vo = val(x - h - 1), vn = val(x + h);
+    const uint32_t vo = val(x - h - 1), vn = val(x + h);
     // first places of values >= vo (vo is among them) and >= vn, side by side
     int lo = 0, hi = w, pl = 0, ph = w;
     while (lo < hi || pl < ph) {
       const int m = min((lo + hi) >> 1, w - 1), q = min((pl + ph) >> 1, w - 1);
-      const float a = W(m), b = W(q);
+      const uint32_t a = W(m), b = W(q);
       if (lo < hi) {
         if (a < vo) lo = m + 1; else hi = m;
       }
@@ -232,19 +237,19 @@ __global__ void __launch_bounds__(VO_MED_T)
     int i = lo;
     if (vn > vo) {
       for (; i + 4 < pl; i += 4) {
-        const float a = W(i + 1), b = W(i + 2), c = W(i + 3), d = W(i + 4);
+        const uint32_t a = W(i + 1), b = W(i + 2), c = W(i + 3), d = W(i + 4);
         W(i) = a, W(i + 1) = b, W(i + 2) = c, W(i + 3) = d;
       }
       for (; i + 1 < pl; i++) W(i) = W(i + 1);
     } else {
       for (; i - 4 >= pl; i -= 4) {
-        const float a = W(i - 1), b = W(i - 2), c = W(i - 3), d = W(i - 4);
+        const uint32_t a = W(i - 1), b = W(i - 2), c = W(i - 3), d = W(i - 4);
         W(i) = a, W(i - 1) = b, W(i - 2) = c, W(i - 3) = d;
       }
       for (; i > pl; i--) W(i) = W(i - 1);
     }
     W(i) = vn;
-    out[((size_t)z * ni + x) * R + r] = W(h);
+    out[((size_t)z * ni + x) * R + r] = fdecode(W(h));
   }
 }
 
@@ -289,7 +294,8 @@ __global__ void __launch_bounds__(32 * DD_SEG)
 }
 
 // Median over w (odd) columns, reflect mode, of the row statistics in[z][x]:
-// each thread finds the value of rank w/2 of its window by counting.  There are
+// each thread finds the value of rank w/2 of its window by counting (NaN last: no
+// value counts that rank where more than half are NaN).  There are
 // too few rows of statistics to fill the chip with sliding windows (vo_median_x
 // took 0.5 ms for 16 rows of 1024), and w^2 comparisons cost a thread 4000 loads.
 __global__ void __launch_bounds__(256)
@@ -302,7 +308,7 @@ __global__ void __launch_bounds__(256)
   const int x = x0 + threadIdx.x;
   if (x >= ni) return;
   const float *v = win + threadIdx.x;
-  float med = v[h];
+  float med = NAN;
   for (int j = 0; j < w; j++) {
     const float c = v[j];
     int lt = 0, le = 0;
