@@ -1,6 +1,7 @@
 """The B-spline prefilter of lprec (the backprojection leaves the coefficients in
-its input) at lengths beside the 32-sample segments, against the float64
-recursion of the same formulas.
+its input) at lengths beside the 32-sample segments and on a line that takes a
+block of more than 512 threads, against the float64 recursion of the same
+formulas.
 
 Bound: each recursion scales an error of the previous sample by 0.27, so a
 coefficient carries a few float32 roundings of values up to 6 times the
@@ -29,7 +30,7 @@ def recursion(x):
 
 
 @pytest.mark.parametrize("n,nproj,nz", [(64, 31, 1), (66, 32, 3), (96, 33, 2), (130, 257, 2),
-                                        (250, 96, 5)])
+                                        (250, 96, 5), (64, 20000, 1)])
 def test_prefilter(cuda, n, nproj, nz):
     import torch
     from tomocupy_b200.reconstruction.lprec import LpRec

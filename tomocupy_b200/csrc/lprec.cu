@@ -158,7 +158,8 @@ __device__ __forceinline__ void pf_fetch(float *dst, const float *src) {  // asy
 }
 __device__ __forceinline__ void pf_fetched() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__global__ void prefilter_rows(float *__restrict__ g, int len, long long nlines) {
+__global__ void __launch_bounds__(1024)
+    prefilter_rows(float *__restrict__ g, int len, long long nlines) {
   extern __shared__ float pf_sm[];
   const int lines = blockDim.y, st = pf_stride(len);
   const long long l0 = (long long)blockIdx.x * lines;
@@ -177,8 +178,8 @@ __global__ void prefilter_rows(float *__restrict__ g, int len, long long nlines)
 // The same along the angles of [nz][len][width]: blockDim.x neighbouring columns
 // of a slice per CTA (64-byte pieces of each row at 16), a thread per segment.
 // The coefficients also go into the layered array that the interpolation reads.
-__global__ void prefilter_cols(float *__restrict__ g, int width, int len,
-                               cudaSurfaceObject_t surf) {
+__global__ void __launch_bounds__(1024)
+    prefilter_cols(float *__restrict__ g, int width, int len, cudaSurfaceObject_t surf) {
   extern __shared__ float pf_sm[];
   const int st = pf_stride(len), c = threadIdx.x;
   const int x = blockIdx.x * blockDim.x + c;
@@ -198,36 +199,7 @@ __global__ void prefilter_cols(float *__restrict__ g, int width, int len,
     }
 }
 
-// Lines that are longer than a CTA's threads or shared memory hold: one thread
-// per line of `len` samples `step` apart, line l starting at (l / per) * outer +
-// (l % per) * inner.
-__global__ void prefilter_serial(float *__restrict__ g, int len, size_t step, long long nlines,
-                                 long long per, size_t outer, size_t inner) {
-  const long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= nlines) return;
-  float *c = g + (size_t)(l / per) * outer + (size_t)(l % per) * inner;
-  const float L = lambda_gain();
-  const int horizon = 12 < len ? 12 : len;
-  float zn = POLE, sum = c[0];
-  for (int k = 0; k < horizon; k++) {
-    sum += zn * c[k * step];
-    zn *= POLE;
-  }
-  float prev = L * sum;
-  c[0] = prev;
-  for (int k = 1; k < len; k++) {
-    prev = L * c[k * step] + POLE * prev;
-    c[k * step] = prev;
-  }
-  prev = (POLE / (POLE - 1.0f)) * c[(size_t)(len - 1) * step];
-  c[(size_t)(len - 1) * step] = prev;
-  for (int k = len - 2; k >= 0; k--) {
-    prev = POLE * (prev - c[k * step]);
-    c[k * step] = prev;
-  }
-}
-
-constexpr int PF_MAX = 32768;  // samples a CTA takes as one line: 1024 segments, 135 KB
+constexpr int PF_MAX = 32768;  // longest line, as for a layered array: 1024 segments, 135 KB
 
 cudaError_t pf_attrs() {
   const int most = 200 * 1024;
@@ -250,8 +222,7 @@ int copy_to_array(cudaArray_t arr, const float *src, int w, int h, int d, cudaSt
 
 // Both passes over g [nz][nproj][n], along the detector, then along the angles,
 // and the result into the layered array.
-int prefilter(float *g, int nz, int nproj, int n, cudaArray_t arr, cudaSurfaceObject_t surf,
-              cudaStream_t s) {
+int prefilter(float *g, int nz, int nproj, int n, cudaSurfaceObject_t surf, cudaStream_t s) {
   const long long nrows = (long long)nz * nproj;
   // as many lines per CTA as 512 threads (1024 along the angles) and 64 KB take
   auto lines = [](int len, int threads, int most) {
@@ -259,23 +230,13 @@ int prefilter(float *g, int nz, int nproj, int n, cudaArray_t arr, cudaSurfaceOb
     while (l > 1 && (l * pf_nseg(len) > threads || l * pf_stride(len) * 4 > 65536)) l /= 2;
     return l;
   };
-  if (n <= PF_MAX) {
-    const int l = lines(n, 512, 16);
-    prefilter_rows<<<ceil_div(nrows, l), dim3(pf_nseg(n), l), (size_t)l * pf_stride(n) * 4, s>>>(
-        g, n, nrows);
-  } else {
-    prefilter_serial<<<ceil_div(nrows, 128), 128, 0, s>>>(g, n, 1, nrows, nrows, 0, n);
-  }
+  int l = lines(n, 512, 16);
+  prefilter_rows<<<ceil_div(nrows, l), dim3(pf_nseg(n), l), (size_t)l * pf_stride(n) * 4, s>>>(
+      g, n, nrows);
   TCB_LAUNCH_CHECK();
-  if (nproj <= PF_MAX) {
-    const int l = lines(nproj, 1024, 16);
-    prefilter_cols<<<dim3(ceil_div(n, l), nz), dim3(l, pf_nseg(nproj)),
-                     (size_t)l * pf_stride(nproj) * 4, s>>>(g, n, nproj, surf);
-  } else {
-    prefilter_serial<<<ceil_div((long long)nz * n, 128), 128, 0, s>>>(
-        g, nproj, n, (long long)nz * n, n, (size_t)nproj * n, 1);
-    if (copy_to_array(arr, g, n, nproj, nz, s) != TCB_OK) return TCB_ERR_CUDA;
-  }
+  l = lines(nproj, 1024, 16);
+  prefilter_cols<<<dim3(ceil_div(n, l), nz), dim3(l, pf_nseg(nproj)),
+                   (size_t)l * pf_stride(nproj) * 4, s>>>(g, n, nproj, surf);
   TCB_LAUNCH_CHECK();
   count_launch(2);
   return TCB_OK;
@@ -572,7 +533,9 @@ extern "C" int tcb_lprec_create(tcb_lprec **out, size_t nproj, size_t nz, size_t
   TCB_CHECK_ARG(nproj >= 2 && nz >= 1 && n >= 2 && ntheta >= 2 && nrho >= 2 &&
                     ntheta % 2 == 0,
                 "tcb_lprec_create: bad sizes");
-  TCB_CHECK_ARG(nz < 2048 && n < 65536 && nproj < 65536, "tcb_lprec_create: sizes too large");
+  // (layered arrays end at 32768 a side, too)
+  TCB_CHECK_ARG(nz < 2048 && n <= (size_t)PF_MAX && nproj <= (size_t)PF_MAX,
+                "tcb_lprec_create: sizes too large");
   TCB_CHECK_ARG(precision == TCB_FLOAT32 || precision == TCB_FLOAT16,
                 "tcb_lprec_create: bad precision %d", precision);
   tcb_lprec *h = new tcb_lprec();
@@ -690,7 +653,7 @@ extern "C" int tcb_lprec_backprojection(tcb_lprec *h, void *f, void *g, void *st
   TCB_CUDA(cudaMemsetAsync(ff, 0, ftot * sizeof(float), s));
   {
     StageTimer st("lprec_prefilter", s);
-    const int rc = prefilter(gf, nz, nproj, n, h->ga, h->surfg, s);
+    const int rc = prefilter(gf, nz, nproj, n, h->surfg, s);
     if (rc != TCB_OK) return rc;
   }
   TCB_CUFFT(cufftSetStream(h->fwd, s));
