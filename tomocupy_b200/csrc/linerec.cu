@@ -387,14 +387,17 @@ __global__ void __launch_bounds__(BX *BY)
 // weights are zero; the sums are bit-identical to backproject_full_tma's.  The
 // other row's two samples enter there times zero, which matters only when they
 // are not finite: where the sum of that row (the neighbouring slice's) is not, its
-// samples are looked through at the end (row_zero; a sum may also overflow).
+// samples are looked through at the end (a sum may also overflow).
 //
 // Z consecutive slices per thread (8, or 4 where that leaves fewer slices
 // unused) share the column arithmetic; rows go in pairs through packed FP32
 // instructions.  Bound: instruction issue, about 20 for the column, 2 (Z + 2)
 // loads and 1.5 (Z + 2) packed operations per angle; the loads alone would allow
 // 3600 updates/ns over the chip at Z = 8.
-// 1024^2 x 16 slices x 720 angles: 4.9 ms, against 15.2 ms for the bilinear form.
+// 1024^2 x 16 slices x 720 angles: 4.7 ms, against 15.2 ms for the bilinear form;
+// 4 slices 1.63.  (Two angles in flight and the registers of three CTAs per SM, as
+// many as fit at Z = 8: with one angle 4.9 and 1.82, with the registers of five
+// 5.3 and 2.04.)
 constexpr int RAC = 16;  // angles per stage
 constexpr float FLOOR_MAGIC = 8388608.f;  // 2^23
 constexpr int FLOOR_BITS = 0x4B000000;    // its bits
@@ -426,11 +429,12 @@ __device__ __forceinline__ unsigned long long lr_lerp2(unsigned long long a, uns
   return r;
 }
 
-// What the samples of a slice's sinogram [nproj][n] that a voxel meets add when they
-// are multiplied by zero: NaN when one of them is not finite, else 0.
-__device__ __noinline__ float row_zero(const float *sino, const float *theta, int nproj, int n,
-                                       float fx, float fy) {
+// Whether one of the samples of a slice's sinogram [nproj][n] that a voxel meets is
+// not finite.
+__device__ __forceinline__ bool row_not_finite(const float *sino, const float *theta, int nproj,
+                                               int n, float fx, float fy) {
   float sum = 0.f;
+#pragma unroll 1
   for (int p = 0; p < nproj; p++) {
     const float u = lr_u(__cosf(theta[p]), __sinf(theta[p]), fx, fy, (float)(n / 2));
     const int ur = (int)(u - 1e-5f);
@@ -438,11 +442,11 @@ __device__ __noinline__ float row_zero(const float *sino, const float *theta, in
     const float *d = sino + (size_t)p * n + ur;
     sum += 0.f * d[0] + 0.f * d[1];
   }
-  return sum;
+  return sum != sum;
 }
 
 template <int Z>
-__global__ void __launch_bounds__(BX *BY, Z == 4 ? 6 : 4)
+__global__ void __launch_bounds__(BX *BY, 3)
     backproject_rows_tma(float *__restrict__ f, const float *__restrict__ data,
                          const __grid_constant__ CUtensorMap map,
                          const float *__restrict__ theta, float c, int sz, int ncz, int n, int nz,
@@ -516,6 +520,7 @@ __global__ void __launch_bounds__(BX *BY, Z == 4 ? 6 : 4)
     if (!ok) break;
     waited = cc + 1;
     auto sum = [&](auto flipped) {
+#pragma unroll 2
       for (int k = 0; k < cnt; k++) {
         const float4 t = s_t[st][k];
         float u = lr_u(t.x, t.y, fx, fy, fh);
@@ -582,6 +587,7 @@ __global__ void __launch_bounds__(BX *BY, Z == 4 ? 6 : 4)
   }
   a[0] = lr_unpack(edge).x;
   a[Z + 1] = lr_unpack(edge).y;
+  unsigned above = 0, below = 0;  // slices whose other row's sum is not finite
 #pragma unroll
   for (int s = 0; s < Z; s++) {
     const int tz = tz0 + s;
@@ -591,14 +597,18 @@ __global__ void __launch_bounds__(BX *BY, Z == 4 ? 6 : 4)
     const int vr = (int)(v - 1e-5f);
     float sum = 0.f;
     if ((vr >= 0) & (vr < nz - 1)) {
-      const int k = (v - vr) > 0.5f ? 0 : 2;  // the other row, v0 + s + k = vr or vr + 1
-      float other = k ? a[s + 2] : a[s];
-      if (!isfinite(other))
-        other = row_zero(data + (size_t)(v0 + s + k) * nproj * n, theta, nproj, n, fx, fy);
-      sum = __fmaf_rn(0.f, other, a[s + 1]);
+      const bool lower = (v - vr) > 0.5f;  // the other row is vr, or vr + 1
+      const float other = lower ? a[s] : a[s + 2];
+      sum = isfinite(other) ? __fmaf_rn(0.f, other, a[s + 1]) : a[s + 1];
+      if (!isfinite(other)) (lower ? below : above) |= 1u << s;
     }
     float *o = f + tx + (size_t)(n - ty - 1) * n + (size_t)tz * n * n;
     *o = __fmaf_rn(sum, c, *o);
+  }
+  for (unsigned left = above | below; left; left &= left - 1) {
+    const int s = __ffs(left) - 1, row = tz0 + s + sz + ((below >> s) & 1 ? -1 : 1);
+    if (row_not_finite(data + (size_t)row * nproj * n, theta, nproj, n, fx, fy))
+      f[tx + (size_t)(n - ty - 1) * n + (size_t)(tz0 + s) * n * n] = NAN;
   }
 }
 
