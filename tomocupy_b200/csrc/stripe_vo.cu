@@ -32,6 +32,7 @@ struct tcb_stripe_vo {
   size_t nproj, nz, ni;
   float snr;
   int la, sm;
+  int la_run, sm_run;        // output columns per thread of the two medians
   float *tt = nullptr;       // [nz][ni][nproj] the chunk with contiguous columns
   float *srt = nullptr;      // [nz][ni][nproj] values sorted along the angles
   int *ids = nullptr;        // [nz][ni][nproj] angle of each sorted value
@@ -46,7 +47,7 @@ namespace tcb {
 namespace {
 
 constexpr int VO_MED_T = 128;  // threads per median block
-constexpr int VO_RUN = 128;    // output columns per median thread
+constexpr int VO_RUN = 128;    // output columns per median thread, at most
 constexpr int VO_MAXW = 127;   // largest median window
 
 __device__ __forceinline__ int reflect_idx(int i, int n) {
@@ -58,18 +59,16 @@ __device__ __forceinline__ int reflect_idx(int i, int n) {
   return m >= n ? p - 1 - m : m;
 }
 
-// Total order of floats as unsigned integers (negative values reversed).
+// Total order of floats as unsigned integers (negative values reversed; a NaN lies
+// beyond the infinity of its sign).
 __device__ __forceinline__ uint32_t fkey(float f) {
   const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
 }
 
 __device__ __forceinline__ float fdecode(uint32_t k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
+  return __uint_as_float(k ^ ((uint32_t)((int32_t)~k >> 31) | 0x80000000u));
 }
-
-// The same with every NaN last: the order that the medians take ranks in.
-__device__ __forceinline__ uint32_t med_key(float f) { return f != f ? 0xFFFFFFFFu : fkey(f); }
 
 // One CTA per column (z, x): the nproj values sorted ascending, ties in angle
 // order; srt/ids [(z * ni + x) * nproj + r].  Stable radix sort of the order bits,
@@ -186,27 +185,27 @@ void sort_columns(const float *tt, int nproj, int ni, int nz, float *srt, int *i
 }
 
 // Median over w (odd) columns, reflect mode, of in[(z * ni + x) * R + r] for
-// every (z, x, r): each thread slides a sorted window along a run of VO_RUN
+// every (z, x, r): each thread slides a sorted window along a run of `len`
 // columns of one (z, r) (window kept interleaved in shared memory).  A chain of
 // dependent shared-memory loads bounds it, so the places of the leaving and of
 // the entering value are searched for together and the values between them move
 // four at a time (one by one, after one search: 1.08 ms for windows of 61 and 21
 // on 16 x 720 x 1024; so 0.58).  The window holds order keys, not floats: a NaN
-// (a pixel with zero flat and dark) has its place too, so the window stays sorted
-// while the NaN passes and after it has left.
+// (0/0 where flat and dark are zero) has its place too, behind all values, so the
+// window stays sorted while the NaN passes and after it has left.
 __global__ void __launch_bounds__(VO_MED_T)
     vo_median_x(const float *__restrict__ in, float *__restrict__ out, int nz, int ni, int R,
-                int w) {
+                int w, int len) {
   extern __shared__ uint32_t wkey[];  // wkey[j * VO_MED_T + t]
   const int t = threadIdx.x;
   const long long g = (long long)blockIdx.x * VO_MED_T + t;
-  const int nrun = (ni + VO_RUN - 1) / VO_RUN;
+  const int nrun = (ni + len - 1) / len;
   if (g >= (long long)nz * nrun * R) return;
   const int r = (int)(g % R);
   const long long q = g / R;
   const int run = (int)(q % nrun), z = (int)(q / nrun);
-  const int x0 = run * VO_RUN, x1 = min(ni, x0 + VO_RUN), h = w / 2;
-  auto val = [&](int x) { return med_key(in[((size_t)z * ni + reflect_idx(x, ni)) * R + r]); };
+  const int x0 = run * len, x1 = min(ni, x0 + len), h = w / 2;
+  auto val = [&](int x) { return fkey(in[((size_t)z * ni + reflect_idx(x, ni)) * R + r]); };
   auto W = [&](int i) -> uint32_t & { return wkey[i * VO_MED_T + t]; };
   for (int j = 0; j < w; j++) {  // insertion sort of the first window
     const uint32_t v = val(x0 - h + j);
@@ -218,8 +217,11 @@ __global__ void __launch_bounds__(VO_MED_T)
     W(i) = v;
   }
   out[((size_t)z * ni + x0) * R + r] = fdecode(W(h));
+  uint32_t next_o = val(x0 - h), next_n = val(x0 + 1 + h);  // loaded a column ahead
   for (int x = x0 + 1; x < x1; x++) {
-    const uint32_t vo = val(x - h - 1), vn = val(x + h);
+    const uint32_t vo = next_o, vn = next_n;
+    next_o = val(x - h);
+    next_n = val(x + 1 + h);
     // first places of values >= vo (vo is among them) and >= vn, side by side
     int lo = 0, hi = w, pl = 0, ph = w;
     while (lo < hi || pl < ph) {
@@ -539,6 +541,22 @@ void vo_release(tcb_stripe_vo *h) {
   h->nbr = nullptr;
 }
 
+// Output columns per thread of vo_median_x: VO_RUN, or where that is less than one
+// wave of blocks, the shortest run that is one (a thread sorts its first window and
+// then slides, and the kernel takes as long as one thread: 16 x 720 x 1024, windows
+// of 61 and 21, runs of 128 0.57 ms, of 94 and 40 0.49; the whole removal of
+// 8 x 360 x 512 0.76 and 0.44 ms).
+int median_run(size_t nz, size_t ni, size_t nproj, int w) {
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, vo_median_x, VO_MED_T,
+                                                    (size_t)w * VO_MED_T * 4) != cudaSuccess) {
+    cudaGetLastError();
+    return VO_RUN;
+  }
+  const size_t fit = (size_t)per * sm_count() * VO_MED_T / (nz * nproj);  // runs of a row
+  return fit * VO_RUN <= ni ? VO_RUN : (int)std::max<size_t>(16, (ni + fit - 1) / fit);
+}
+
 int pow2_at_least(int v) {
   int p = 1;
   while (p < v) p <<= 1;
@@ -599,6 +617,8 @@ extern "C" int tcb_stripe_vo_create(tcb_stripe_vo **out, size_t nproj, size_t nz
     set_error("tcb_stripe_vo_create: shared-memory attribute failed");
     return TCB_ERR_CUDA;
   }
+  h->la_run = median_run(nz, ni, nproj, la_size);
+  h->sm_run = median_run(nz, ni, nproj, sm_size);
   *out = h;
   return TCB_OK;
 }
@@ -620,11 +640,11 @@ extern "C" int tcb_stripe_vo_apply(tcb_stripe_vo *h, float *tomo, size_t pstride
   // sorts read the column-contiguous copy tt
   auto sort_cols = [&]() { sort_columns(h->tt, np, ni, nz, h->srt, h->ids, s); };
   const dim3 tgrid(ceil_div(h->ni, 32), ceil_div(h->nproj, 32), nz), tblk(32, 8);
-  auto median = [&](const float *in, float *outp, int R, int w) {
-    const int nrun = (ni + VO_RUN - 1) / VO_RUN;
+  auto median = [&](const float *in, float *outp, int R, int w, int run) {
+    const int nrun = (ni + run - 1) / run;
     const long long thr = (long long)nz * nrun * R;
     vo_median_x<<<(unsigned)((thr + VO_MED_T - 1) / VO_MED_T), VO_MED_T,
-                  (size_t)w * VO_MED_T * 4, s>>>(in, outp, nz, ni, R, w);
+                  (size_t)w * VO_MED_T * 4, s>>>(in, outp, nz, ni, R, w, run);
   };
   StageTimer t("stripe_vo", s);
   // 1. dead stripes
@@ -646,7 +666,7 @@ extern "C" int tcb_stripe_vo_apply(tcb_stripe_vo *h, float *tomo, size_t pstride
   }
   {
     StageTimer st("stripe_vo_median", s);
-    median(h->srt, h->smooth, np, h->la);
+    median(h->srt, h->smooth, np, h->la, h->la_run);
   }
   const size_t vals = (size_t)nz * ni * np;
   {
@@ -669,7 +689,7 @@ extern "C" int tcb_stripe_vo_apply(tcb_stripe_vo *h, float *tomo, size_t pstride
   }
   {
     StageTimer st("stripe_vo_median", s);
-    median(h->srt, h->smooth, np, h->sm);
+    median(h->srt, h->smooth, np, h->sm, h->sm_run);
   }
   {
     StageTimer st("stripe_vo_unsort", s);
