@@ -50,8 +50,8 @@ class BackprojLamFourierParallel:
             self.nthetac, self.dethc)
         # filter applied along the rows of each projection (not sinograms); center
         # and wfilter may be changed between calls
-        self.wfilter = torch.as_tensor(fbp_filter.calc_filter(self.ne, args.fbp_filter),
-                                       device=self.device)
+        wfilter = fbp_filter.calc_filter(self.ne, args.fbp_filter)
+        self.wfilter = torch.as_tensor(wfilter, device=self.device)
         self.pad = self.ne // 2 - self.detw // 2
         self.t = rfftfreq32(self.ne, self.device)
         self._crop = torch.empty((self.nthetac, self.deth, self.detw), dtype=torch.float32,
@@ -70,7 +70,7 @@ class BackprojLamFourierParallel:
         self._can_fuse = (fftfilter.supported(self.detw) and self.nthetac % 2 == 0
                           and args.dtype != "float16")
         self._dtype = args.dtype
-        if self._fused() is None:
+        if self._fused(wfilter) is None:
             self._padded()
         self.cl_writer = cl_writer
         self.rec_fun = self.rec_lam
@@ -80,12 +80,14 @@ class BackprojLamFourierParallel:
         """The filter on padded rows (cuFFT plans of length 4 detw)."""
         return fbp_filter.FBPFilter(self.ne, self.deth, self.nthetac, self._dtype)
 
-    def _fused(self):
-        """The fused filter for the present ``center`` and ``wfilter``, or None
-        where the padded chain has to run."""
+    def _fused(self, wf=None):
+        """The fused filter for the present ``center`` and ``wfilter`` (``wf``: its
+        values, where the caller has them on the host), or None where the padded
+        chain has to run."""
         if not self._can_fuse or not float(self.center - self.detw / 2).is_integer():
             return None
-        wf = self.wfilter.detach().cpu().numpy().copy()
+        if wf is None:
+            wf = self.wfilter.detach().cpu().numpy().copy()
         if (wf.shape != (self.ne // 2 + 1,) or wf.dtype != np.float32
                 or not np.isfinite(wf).all()):
             return None
