@@ -214,10 +214,12 @@ __global__ void sfb_rows(const float *__restrict__ in, int H, int Wi, float *__r
 // comes with the taps so that the compiler does not know it.
 // These instructions (two cycles of the FP32 pipe each) are the bound: 0.13 ms per
 // pass over the 7 levels of 16 slices of 1500 x 2048 at 32 taps.  Measured there,
-// one output at a time and packed: analysis rows 0.45 and 0.44 ms, columns 0.40
-// and 0.36, synthesis columns 0.51 and 0.33, rows 0.41 and 0.40; what is left is
+// one output at a time and packed: analysis rows 0.43 and 0.40 ms, columns 0.39
+// and 0.34, synthesis columns 0.49 and 0.30, rows 0.39 and 0.35; what is left is
 // the staging's latency (rows) and the few warps 127 registers leave (columns of the
 // analysis; the synthesis gains from three blocks per SM at 80: 0.36 with two).
+// The small levels are latency: 2 slices of 360 x 512 take 0.21 ms, 0.23 one output
+// at a time, of the call's 0.26 and 0.28.
 struct TapPair {
   float4 c[MAXL];  // (a, a, b, b) of tap k
   float2 nz;       // -0, -0
@@ -331,7 +333,7 @@ __device__ __forceinline__ void store_rows(float *buf, Value value, int e0, int 
   }
 }
 
-constexpr int FB_PAIRS = 16;  // pairs of rows per block, at most
+constexpr int FB_PAIRS = 2;  // pairs of rows per block, at most
 
 // Shared memory places of a row of n staged samples, one skipped after every g
 // (an even count: the buffers behind are read in 16-byte pieces).
@@ -683,22 +685,34 @@ struct tcb_stripe_fw {
 };
 
 namespace {
-// outputs per thread: of the analysis along the rows, along the columns, and half
-// of the synthesis'
+// Outputs per thread of the analysis along the rows; the largest count along the
+// columns, and of the synthesis half of it.
 constexpr int FB_RO = 4, FB_CO = 8, FB_M = 4;
+// Fewer outputs of a kernel in a level than this leave most of the chip idle, and
+// what counts is how long one thread takes: half as many outputs per thread then.
+// Measured over 512 to 2048 columns, 360 to 1500 angles, 2 to 16 slices, at the
+// full and at half the count: analysis of columns 10.5 and 7.5 us at 10^5
+// outputs, 14.0 and 14.2 at 1.6 10^6, 28.4 and 31.1 at 5.6 10^6; synthesis of
+// columns 5.3 and 4.4, 6.9 and 6.6 at 5 10^5, 11.4 and 12.5; of rows 5.3 and 4.6,
+// 7.0 and 5.6 at 4 10^5, 9.8 and 10.1 at 1.1 10^6, 25.2 and 26.1.
+constexpr long long FB_AC_FEW = 1500000, FB_SC_FEW = 500000, FB_SR_FEW = 1000000;
 // wide rows' shared memory (one value for every call: threads may launch at once)
 constexpr int FB_MAX_SMEM = 220 * 1024;
 
 // Pairs of rows and threads per block of a row kernel: `groups` threads' turns and
-// `bytes` of shared memory per pair.  The split that leaves the fewest lanes idle
-// in the last turn, the smaller block where they are alike.
-void rows_split(int groups, size_t bytes, int &RB, int &T) {
+// `bytes` of shared memory per pair, `pairs` in all.  A block stages its pairs one
+// after the other, so it takes one, or two where that leaves a block per SM and
+// fewer lanes idle in the last turn; the smaller block where they are alike.  (Up
+// to 16 pairs, chosen by the idle lanes alone: 10 to 15 us for the small levels,
+// which take 4.5 so, and 190 against 171 us for 1690 x 1290 x 16.)
+void rows_split(int groups, size_t bytes, long long pairs, int &RB, int &T) {
+  const int most = pairs >= 2 * sm_count() ? FB_PAIRS : 1;
   double best = 0;
-  for (int rb = 1; rb <= FB_PAIRS && (rb == 1 || rb * bytes <= 40960); rb++)
+  for (int rb = 1; rb <= most && (rb == 1 || rb * bytes <= 40960); rb++)
     for (int th = 128; th <= 320; th += 32) {
       const int turns = (rb * groups + th - 1) / th;
       const double use = (double)rb * groups / ((double)turns * th);
-      if (use > best + 0.02) best = use, RB = rb, T = th;
+      if (best == 0 || use > best + 0.02) best = use, RB = rb, T = th;
     }
 }
 
@@ -708,7 +722,7 @@ void launch_afb_rows(const tcb_stripe_fw *h, const float *x, long long xsz, int 
   const int ngrp = (Wo + FB_RO - 1) / FB_RO;
   const size_t bytes = (size_t)fw_pad(2 * FB_RO * ngrp + L - 2, 2 * FB_RO) * sizeof(f32x2);
   int RB, T;
-  rows_split(ngrp, bytes, RB, T);
+  rows_split(ngrp, bytes, ((long long)B * Hk + 1) / 2, RB, T);
   const size_t smem = RB * bytes + (size_t)T * 4 * FB_RO * sizeof(float);
   if (smem > 40960)
     cudaFuncSetAttribute(afb_rows_t<L, FB_RO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -718,37 +732,62 @@ void launch_afb_rows(const tcb_stripe_fw *h, const float *x, long long xsz, int 
                                                      h->ana);
 }
 
+template <int L, int RO>
+void afb_cols_of(const tcb_stripe_fw *h, float *out, int B, int Hk, int Wo, int Ho, int padl,
+                 cudaStream_t s) {
+  const long long nb = (long long)ceil_div(Wo, 64) * (2LL * B) * ((Ho + 8 * RO - 1) / (8 * RO));
+  afb_cols_t<L, RO><<<(unsigned)nb, 256, 0, s>>>(h->tmp, out, B, Hk, Wo, Ho, padl, h->ana);
+}
+
 template <int L>
 void launch_afb_cols(const tcb_stripe_fw *h, float *out, int B, int Hk, int Wo, int Ho, int padl,
                      cudaStream_t s) {
-  const long long nb = (long long)ceil_div(Wo, 64) * (2LL * B) *
-                       ((Ho + 8 * FB_CO - 1) / (8 * FB_CO));
-  afb_cols_t<L, FB_CO><<<(unsigned)nb, 256, 0, s>>>(h->tmp, out, B, Hk, Wo, Ho, padl, h->ana);
+  if (4LL * B * Ho * Wo < FB_AC_FEW)
+    afb_cols_of<L, FB_CO / 2>(h, out, B, Hk, Wo, Ho, padl, s);
+  else
+    afb_cols_of<L, FB_CO>(h, out, B, Hk, Wo, Ho, padl, s);
+}
+
+template <int L, int M>
+void sfb_cols_of(const tcb_stripe_fw *h, const float *y, int Hi, int Wi, int B, int Hc,
+                 cudaStream_t s) {
+  const long long nb = (long long)ceil_div(Wi, 64) * (2LL * B) * ((Hc + 16 * M - 1) / (16 * M));
+  sfb_cols_t<L, M><<<(unsigned)nb, 256, 0, s>>>(y, 4LL * Hi * Wi, Hi, Wi, Wi, h->tmp, B, Hc,
+                                                h->syn);
 }
 
 template <int L>
 void launch_sfb_cols(const tcb_stripe_fw *h, const float *y, int Hi, int Wi, int B, int Hc,
                      cudaStream_t s) {
-  const long long nb = (long long)ceil_div(Wi, 64) * (2LL * B) *
-                       ((Hc + 16 * FB_M - 1) / (16 * FB_M));
-  sfb_cols_t<L, FB_M><<<(unsigned)nb, 256, 0, s>>>(y, 4LL * Hi * Wi, Hi, Wi, Wi, h->tmp, B, Hc,
-                                                   h->syn);
+  if (2LL * B * Hc * Wi < FB_SC_FEW)
+    sfb_cols_of<L, FB_M / 2>(h, y, Hi, Wi, B, Hc, s);
+  else
+    sfb_cols_of<L, FB_M>(h, y, Hi, Wi, B, Hc, s);
+}
+
+template <int L, int M>
+void sfb_rows_of(const tcb_stripe_fw *h, int Hc, int Wi, float *dst, long long dsz, int Wd,
+                 int Hrows, int B, cudaStream_t s) {
+  const int ngrp = (Wd + 2 * M - 1) / (2 * M);
+  const size_t bytes = (size_t)fw_pad(M * ngrp + L / 2 - 1, M) * sizeof(ulonglong2);
+  int RB, T;
+  rows_split(ngrp, bytes, ((long long)B * Hrows + 1) / 2, RB, T);
+  const size_t smem = RB * bytes + (size_t)T * 4 * M * sizeof(float);
+  if (smem > 40960)
+    cudaFuncSetAttribute(sfb_rows_t<L, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         FB_MAX_SMEM);
+  const long long nb = ((long long)B * Hrows + 2 * RB - 1) / (2 * RB);
+  sfb_rows_t<L, M><<<(unsigned)nb, T, smem, s>>>(h->tmp, Hc, Wi, dst, dsz, Wd, Hrows, Wd, B, RB,
+                                                 h->syn);
 }
 
 template <int L>
 void launch_sfb_rows(const tcb_stripe_fw *h, int Hc, int Wi, float *dst, long long dsz, int Wd,
                      int Hrows, int B, cudaStream_t s) {
-  const int ngrp = (Wd + 2 * FB_M - 1) / (2 * FB_M);
-  const size_t bytes = (size_t)fw_pad(FB_M * ngrp + L / 2 - 1, FB_M) * sizeof(ulonglong2);
-  int RB, T;
-  rows_split(ngrp, bytes, RB, T);
-  const size_t smem = RB * bytes + (size_t)T * 4 * FB_M * sizeof(float);
-  if (smem > 40960)
-    cudaFuncSetAttribute(sfb_rows_t<L, FB_M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         FB_MAX_SMEM);
-  const long long nb = ((long long)B * Hrows + 2 * RB - 1) / (2 * RB);
-  sfb_rows_t<L, FB_M><<<(unsigned)nb, T, smem, s>>>(h->tmp, Hc, Wi, dst, dsz, Wd, Hrows, Wd, B, RB,
-                                                    h->syn);
+  if ((long long)B * Hrows * Wd < FB_SR_FEW)
+    sfb_rows_of<L, FB_M / 2>(h, Hc, Wi, dst, dsz, Wd, Hrows, B, s);
+  else
+    sfb_rows_of<L, FB_M>(h, Hc, Wi, dst, dsz, Wd, Hrows, B, s);
 }
 
 bool blocked_length(int L) { return L == 2 || L == 10 || L == 32; }
