@@ -376,9 +376,9 @@ int tcb_fourierrec_backprojection_slices(tcb_fourierrec *h, void *f, void *g,
  * backproj_functions.py:107). */
 int tcb_fourierrec_pack(tcb_fourierrec *h, void *g, const void *src,
                         size_t row_stride, size_t xoff, void *stream);
-/* Tuning knob (no reference counterpart): slice pairs accumulated per
- * gridding block, 2/4/8 (16 is accepted and acts as 8), or 0 for the largest
- * that the handle's nz allows.
+/* Tuning knob (no reference counterpart): the most slice pairs that a gridding
+ * block accumulates, 2/4/8 (16 is accepted and acts as 8), or 0 for the
+ * library's choice; within that the cheapest cover of the handle's nz is taken.
  * Results do not depend on it beyond fp32 summation order. */
 int tcb_fourierrec_set_pairs_per_block(tcb_fourierrec *h, int pairs);
 /* Gridding mode (no reference counterpart).  TCB_GRID_FP32: the fp32

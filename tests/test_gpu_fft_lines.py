@@ -43,3 +43,52 @@ def test_lines_vs_full_transform(cuda, monkeypatch, n, nproj, nz):
     want = _run(*args, {"TCB_FOURIERREC_FULL_FFT2D": "1"})
     assert rel_l2(_run(*args, {}), want) < 1e-6
     assert rel_l2(_run(*args, {"TCB_FOURIERREC_FFT": "cufft"}), want) < 1e-6
+
+
+def test_little_memory(cuda):
+    """A handle is created as soon as what it cannot do without fits (the copy for
+    the columns is given up), and gives the same images.  2n = 4 * 1223, for which
+    cuFFT takes a workspace larger than the grid."""
+    import torch
+    from tomocupy_b200 import _lib
+    from tomocupy_b200.cfunc_fourierrec import cfunc_fourierrec
+    n, nproj, nz = 2446, 8, 8
+    theta = torch.as_tensor((np.arange(nproj) * np.pi / nproj + 0.01).astype(np.float32),
+                            device=cuda)
+    g = torch.randn((nz, nproj, n, 2), generator=torch.Generator(device=cuda).manual_seed(1),
+                    device=cuda)
+    f, gc = torch.empty((nz, n, n, 2), device=cuda), torch.empty_like(g)
+
+    def run(budget=None):
+        """Bytes that a handle takes where `budget` are free (None: it is refused)."""
+        torch.cuda.empty_cache()
+        hold = None
+        if budget is not None:
+            hold = torch.empty(torch.cuda.mem_get_info()[0] - budget, dtype=torch.uint8,
+                               device=cuda)
+        before = torch.cuda.mem_get_info()[0]
+        try:
+            op = cfunc_fourierrec(nproj, nz, n, theta)
+        except _lib.TcbError:
+            return None
+        finally:
+            used = before - torch.cuda.mem_get_info()[0]
+            del hold
+            torch.cuda.empty_cache()
+        gc.copy_(g)
+        op.backprojection(f, gc, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        op.free()
+        return used
+
+    mb = 1 << 20
+    lo, hi = nz * 4 * n * n * 8, run() + 64 * mb
+    want = f.cpu().numpy()
+    while hi - lo > 48 * mb:
+        mid = (lo + hi) // 2 // mb * mb
+        if run(mid) is None:
+            lo = mid
+        else:
+            hi = mid
+    assert hi - run(hi) < 160 * mb
+    assert rel_l2(f.cpu().numpy(), want) < 1e-6

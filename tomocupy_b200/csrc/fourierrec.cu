@@ -308,8 +308,8 @@ __device__ __forceinline__ int tile_origin(int f, int origin, int twon) {
 // loads); the next 256 samples are located and their values loaded meanwhile.
 // Sums run in the list's order.
 //
-// Bound: instruction issue; the FP32 pipe alone would take 4 cell sums per
-// useful one ((8 + 8)^2 cells of 8 x 8 blocks reach a sample).  8 x 8 cells per
+// Bound: instruction issue; a footprint of 9 meets two blocks of 8 per axis on
+// average, 256 cell sums for 81 useful ones.  8 x 8 cells per
 // warp cost 16 + 6 / Z lane-FMAs per pair and sample against 36 at 16 x 16;
 // 8 x 4 (12) spend it again on loading the values.  8 pairs: 0.10 ms at 512 x
 // 360, 0.29 ms at 1024 x 720, 1.15 ms at 2048 x 1500; one cell per lane, samples
@@ -2160,7 +2160,7 @@ int build_lists(tcb_fourierrec *h) {
       break;
     }
     // items, longest first (then in tile order)
-    const long long len = std::max<long long>(1024, ntot / (8 * 148) / GS * GS);
+    const long long len = std::max<long long>(1024, ntot / (8LL * sm_count()) / GS * GS);
     std::vector<GridItem> items;
     std::vector<GridSplit> splits;
     int slots = 0;
@@ -2523,29 +2523,37 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
   }
   if (r == CUFFT_SUCCESS && !h->pruned)
     r = cufftPlanMany(&h->plan2d, 2, len2, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, (int)nz);
-  if (h->pruned && !h->own_n) {
-    // the columns on a transposed copy; within the grid when the copy does not fit
-    if (cudaMalloc(&h->t1, nz * n * N2 * sizeof(float2)) != cudaSuccess) {
-      cudaGetLastError();
-      h->t1 = nullptr;
-    }
+  // the columns on a transposed copy, if that fits beside what has to
+  auto copy = [&]() {
+    if (cudaMalloc(&h->t1, nz * n * N2 * sizeof(float2)) == cudaSuccess) return true;
+    cudaGetLastError();
+    h->t1 = nullptr;
+    return false;
+  };
+  auto no_copy = [&]() {
+    cudaGetLastError();
+    cudaFree(h->t1);
+    h->t1 = nullptr;
+  };
+  if (r == CUFFT_SUCCESS && h->pruned && !h->own_n && own_sel && N2 <= (size_t)mixfft::MAX_N) {
     // 2n a product of primes up to 17 (8 pairs at 4896 =
     // 17 18 16: 1.73 ms with the copy between the passes; cuFFT's passes 4.9)
     std::vector<float2> twh;
-    if (h->t1 && own_sel && N2 <= (size_t)mixfft::MAX_N) h->mix = mixfft::make_plan((int)N2, twh);
-    if (h->mix.n) {
+    const mixfft::Plan mix = mixfft::make_plan((int)N2, twh);
+    if (mix.n && copy()) {
       if (cudaMalloc(&h->mixtw, twh.size() * sizeof(float2)) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("tcb_fourierrec_create: out of device memory for the FFT tables");
-        return fail(TCB_ERR_OUT_OF_MEMORY);
-      }
-      e = cudaMemcpy(h->mixtw, twh.data(), twh.size() * sizeof(float2), cudaMemcpyHostToDevice);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mixfft::ifft_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)mixfft::smem_bytes(mixfft::MAX_N));
-      if (e != cudaSuccess) {
-        set_error("tcb_fourierrec_create: FFT setup failed: %s", cudaGetErrorString(e));
-        return fail(TCB_ERR_CUDA);
+        h->mixtw = nullptr;
+        no_copy();
+      } else {
+        e = cudaMemcpy(h->mixtw, twh.data(), twh.size() * sizeof(float2), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(mixfft::ifft_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)mixfft::smem_bytes(mixfft::MAX_N));
+        if (e != cudaSuccess) {
+          set_error("tcb_fourierrec_create: FFT setup failed: %s", cudaGetErrorString(e));
+          return fail(TCB_ERR_CUDA);
+        }
+        h->mix = mix;
       }
     }
   }
@@ -2553,13 +2561,11 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
     int lr[1] = {(int)(2 * n)};
     r = cufftPlanMany(&h->plan_rows, 1, lr, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
                       (int)(2 * n * nz));
-    if (r == CUFFT_SUCCESS && h->t1 &&
+    if (r == CUFFT_SUCCESS && copy() &&
         cufftPlanMany(&h->plan_cols, 1, lr, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
                       (int)(n * nz)) != CUFFT_SUCCESS) {
       // no room for this plan's workspace beside the copy
-      cudaGetLastError();
-      cudaFree(h->t1);
-      h->t1 = nullptr;
+      no_copy();
       h->plan_cols = 0;
     }
     int emb[1] = {(int)(2 * n)};
