@@ -37,6 +37,22 @@ def ref():
     return refglue
 
 
+@pytest.fixture(params=["auto", "tensor"])
+def gridding(request, monkeypatch):
+    """fourierrec's gridding in the drivers: as the automatic rule chooses it (fp32
+    registers at the few slices of a test), and on the tensor cores with streamed
+    weights, which the rule takes for larger chunks."""
+    if request.param == "tensor":
+        from tomocupy_b200.pipeline import SinoPipeline
+        choose = SinoPipeline._set_gridding
+
+        def tensor(self, gridding, precision):
+            return choose(self, "tensor_stream" if precision == "mixed" else "tensor_fp32",
+                          precision)
+        monkeypatch.setattr(SinoPipeline, "_set_gridding", tensor)
+    return request.param
+
+
 class TorchCuFFT:
     """Real FFTs through cuFFT (torch.fft on the GPU), the library that the
     reference's cupy.fft calls, with NumPy's types (float32 <-> complex64,

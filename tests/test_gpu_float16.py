@@ -4,9 +4,9 @@ With dtype 'float16' the reference crops the projections to the centred
 power-of-two width and shifts the centre (dataio/reader.py:155-165), takes a
 power-of-two filter length (reconstruction/backproj_functions.py:52-54) and
 runs its cfunc_*fp16 operators, writing float16 volumes.  Here the same
-sizes and centre, fp16 output slices, fourierrec on the mixed-precision
-(fp16 weights and values, fp32 accumulation) gridding, lprec and linerec
-accumulating in fp32.  Budget: rel-L2 <= 2e-3 against the FP64 oracle (the
+sizes and centre, fp16 output slices, fourierrec on the mixed-precision path
+(from 9 slice pairs fp16 weights and values with fp32 accumulation, below in fp32
+registers; both are run here), lprec and linerec accumulating in fp32.  Budget: rel-L2 <= 2e-3 against the FP64 oracle (the
 fp16 rounding of the output alone is ~3e-4)."""
 import numpy as np
 import pytest
@@ -35,7 +35,7 @@ def _run(driver, data, dark, flat, theta, **opts):
 
 
 @pytest.mark.parametrize("driver", ["all", "steps"])
-def test_float16_fourierrec_crop_and_centre(cuda, driver):
+def test_float16_fourierrec_crop_and_centre(cuda, driver, gridding):
     """ni = 300 columns -> the centred 256 (columns 22..277), centre 150 -> 128;
     the float16 volume against the FP64 oracle on those columns."""
     from oracle import np_tomo

@@ -64,6 +64,20 @@ def test_tensor_fp32_gridding_vs_reference(cuda, ref, n, nproj, nz, kind):
     assert rel_l2(ours, fp32) < 1e-5
 
 
+@pytest.mark.parametrize("n,nproj,nz,kind", CASES + [(256, 301, 32, "uniform"),
+                                                      (1024, 90, 64, "uniform")])
+def test_tensor_fp32_gridding_vs_registers(cuda, n, nproj, nz, kind):
+    """The split-fp16 form against the fp32 registers (which test_gpu_gridding_regs.py
+    compares with float64), both group sizes (64 and 128 columns), one and two
+    producer warps."""
+    from tomocupy_b200 import _lib
+    theta = torch.as_tensor(_theta(nproj, kind, seed=n), device=cuda)
+    g = torch.randn((nz, nproj, n, 2), device=cuda)
+    ours = _run(cuda, n, nproj, nz, theta, g, _lib.GRID_TENSOR_FP32)
+    assert torch.isfinite(ours).all()
+    assert rel_l2(ours, _run(cuda, n, nproj, nz, theta, g, _lib.GRID_FP32)) < 1e-5
+
+
 @pytest.mark.parametrize("n,nproj,nz", [(128, 90, 2), (512, 360, 40), (2048, 150, 2)])
 def test_tensor_stream_mixed_vs_fp32(cuda, n, nproj, nz):
     from tomocupy_b200 import _lib

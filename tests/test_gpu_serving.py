@@ -108,9 +108,8 @@ def test_request_matches_gpurec(cuda):
     writer = ArrayWriter(device="cpu", pin=True)
     GPURec(ArrayReader(req.frames, req.dark, req.flat, theta=req.theta, pin=True),
            writer).recon_all()
-    # the server grids with the fp32 register kernel (no per-geometry weight
-    # tables), GPURec on the tensor cores with streamed weights: the two agree
-    # within the fourierrec tolerance
+    # both grid these chunks of 8 rows in fp32 registers, the server as one of a
+    # stream's chunks: they agree within the fourierrec tolerance
     assert rel_l2(req.out, writer.rec) < 1e-5
 
 

@@ -45,7 +45,7 @@ def _sweep(one_slice, precision, shifts, ncz=4, pairs=0, graph=True):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["float32", "mixed"])
-def test_graph_replay_equals_eager(cuda, one_slice, precision):
+def test_graph_replay_equals_eager(cuda, one_slice, precision, gridding):
     shifts = np.arange(-5, 5) * 0.75
     _, eager = _sweep(one_slice, precision, shifts, graph=False)
     sw, graph = _sweep(one_slice, precision, shifts, graph=True)
@@ -56,7 +56,7 @@ def test_graph_replay_equals_eager(cuda, one_slice, precision):
 
 
 @pytest.mark.gpu
-def test_mixed_sweep_vs_fp64_oracle_per_center(cuda, one_slice):
+def test_mixed_sweep_vs_fp64_oracle_per_center(cuda, one_slice, gridding):
     from oracle import np_tomo
     from tomocupy_b200.trycenter import per_center_errors
     shifts = np.array([-3.0, -1.5, -0.375, 0.0, 1.125, 2.5])

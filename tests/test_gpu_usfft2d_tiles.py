@@ -1,7 +1,8 @@
 """The output-stationary adjoint gridding of usfft2d at the sizes where its
 tiling can go wrong, against the float64 restatement: the smallest grid, grids
 that are no multiple of the 64 x 32 cells of a CTA, angle counts beside the 256
-of one search, widths that leave partly filled groups of 128 candidates.
+of a search by one angle per thread (border tiles) and the 1024 of one by four
+(the others), widths that leave partly filled groups of 256 candidates.
 
 Bound: a cell sums at most a few thousand float32 products in one order
 (relative error below 1e-6 of the sum of their magnitudes), the sample positions
@@ -20,7 +21,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,ntheta,deth,nrows", [
-    (64, 7, 64, 33), (66, 255, 12, 7), (80, 257, 10, 6), (98, 1, 8, 5), (130, 40, 6, 4)])
+    (64, 7, 64, 33), (66, 255, 12, 7), (80, 257, 10, 6), (98, 1, 8, 5), (130, 40, 6, 4),
+    (130, 1023, 2, 2), (98, 1030, 2, 2)])
 def test_usfft2d_adj_rows_vs_float64(cuda, n, ntheta, deth, nrows):
     import torch
     from tomocupy_b200.cfunc_usfft2d import cfunc_usfft2d

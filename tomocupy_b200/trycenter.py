@@ -188,7 +188,7 @@ def autotune(n, nproj, theta, center, shifts, data, dark0=None, flat0=None, *,
     candidates: iterable of (ncz, pairs_per_block); by default chunk sizes
     32..128 when the geometry's gridding runs on the tensor cores with
     streamed weights (pairs_per_block does not apply there), else chunk sizes
-    8..64 with register-gridding depths 4..16 pairs.  Returns {"ncz",
+    8..64 with register-gridding depths of 4 and 8 pairs.  Returns {"ncz",
     "pairs_per_block", "ms", "table"}; results are cached per geometry
     in-process and, when cache_file is given, in that JSON file.
     """
@@ -208,7 +208,7 @@ def autotune(n, nproj, theta, center, shifts, data, dark0=None, flat0=None, *,
         if first.pipe.gridding in (_lib.GRID_TENSOR_FP32, _lib.GRID_TENSOR_STREAM):
             candidates = [(64, 0), (32, 0), (128, 0)]
         else:
-            candidates = [(ncz, zb) for ncz in (8, 16, 32, 64) for zb in (4, 8, 16)
+            candidates = [(ncz, zb) for ncz in (8, 16, 32, 64) for zb in (4, 8)
                           if zb <= ncz // 2]
             first.free()
             first = None
