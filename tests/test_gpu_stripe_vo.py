@@ -46,6 +46,17 @@ def test_vo_default_windows_vs_oracle(cuda, nproj, nz, ni):
     assert err < 1e-5, err
 
 
+def test_vo_operators_of_different_widths_side_by_side(cuda):
+    """A wide operator still runs after a narrow one was made."""
+    from tomocupy_b200.processing.remove_stripe import remove_all_stripe
+    _, vo_input = _cases()
+    wide = torch.as_tensor(vo_input(24, 1, 6000, seed=1), device=cuda)
+    narrow = torch.as_tensor(vo_input(24, 1, 100, seed=2), device=cuda)
+    first = remove_all_stripe(wide.clone(), 3.0, 31, 11)
+    remove_all_stripe(narrow, 3.0, 31, 11)
+    assert torch.equal(remove_all_stripe(wide.clone(), 3.0, 31, 11), first)
+
+
 def test_vo_fused_driver_matches_reference_chain(cuda, ref):
     """dark/flat -> Vo's ring removal -> -log -> filter -> fourierrec in
     GPURec.recon_all against the restated ring removal feeding the

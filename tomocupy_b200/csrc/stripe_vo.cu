@@ -49,6 +49,7 @@ namespace {
 constexpr int VO_MED_T = 128;  // threads per median block
 constexpr int VO_RUN = 128;    // output columns per median thread, at most
 constexpr int VO_MAXW = 127;   // largest median window
+constexpr int VO_MAXNI = 8192; // widest row
 
 __device__ __forceinline__ int reflect_idx(int i, int n) {
   // scipy.ndimage mode 'reflect' (d c b a | a b c d | d c b a)
@@ -573,9 +574,9 @@ extern "C" int tcb_stripe_vo_create(tcb_stripe_vo **out, size_t nproj, size_t nz
   TCB_CHECK_ARG(out, "tcb_stripe_vo_create: null out");
   *out = nullptr;
   TCB_CHECK_ARG(nproj >= 12 && nproj <= 8192 && nz >= 1 && nz <= 65535 && ni >= 8 &&
-                    ni <= 8192,
-                "tcb_stripe_vo_create: sizes nproj=%zu (12..8192), nz=%zu, ni=%zu (8..8192)",
-                nproj, nz, ni);
+                    ni <= (size_t)VO_MAXNI,
+                "tcb_stripe_vo_create: sizes nproj=%zu (12..8192), nz=%zu, ni=%zu (8..%d)",
+                nproj, nz, ni, VO_MAXNI);
   TCB_CHECK_ARG(la_size >= 1 && la_size <= VO_MAXW && la_size % 2 == 1 && sm_size >= 1 &&
                     sm_size <= VO_MAXW && sm_size % 2 == 1,
                 "tcb_stripe_vo_create: median windows must be odd and <= %d (got %d, %d)",
@@ -605,13 +606,15 @@ extern "C" int tcb_stripe_vo_create(tcb_stripe_vo **out, size_t nproj, size_t nz
     set_error("tcb_stripe_vo_create: out of device memory");
     return TCB_ERR_OUT_OF_MEMORY;
   }
-  const int med_smem = VO_MAXW * VO_MED_T * 4;
+  // the largest sizes, not this handle's: the attributes belong to the kernels, and
+  // handles of other sizes are in use at the same time
+  const int med_smem = VO_MAXW * VO_MED_T * 4, det_smem = 3 * VO_MAXNI * 4;
   if (cudaFuncSetAttribute(vo_sort_cols<VS_MAXE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            VS_MAXE * VS_T * 6) != cudaSuccess ||
       cudaFuncSetAttribute(vo_median_x, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            med_smem) != cudaSuccess ||
       cudaFuncSetAttribute(vo_detect, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(2 * ni * 4 + pow2_at_least((int)ni) * 4)) != cudaSuccess) {
+                           det_smem) != cudaSuccess) {
     vo_release(h);
     delete h;
     set_error("tcb_stripe_vo_create: shared-memory attribute failed");
