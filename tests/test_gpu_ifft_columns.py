@@ -1,9 +1,9 @@
-"""fourierrec's inverse transform of widths that are no powers of two: the
-mixed-radix lines at every radix (3 .. 18) and count of stages, and cuFFT on the
-transposed columns, against one full cuFFT transform of the same grid.
+"""fourierrec's inverse transform of widths that are no powers of two: cuFFT on the
+rows and then on the kept columns, transposed or within the grid, against one full
+cuFFT transform of the same grid.
 
-Bound: each stage rounds a value a few times (2^-24 relative), four stages in
-either transform: below 1e-6 of the result's norm."""
+Bound: a transform of these lengths rounds a value a few times at each of its
+stages (2^-24 relative): below 1e-6 of the result's norm."""
 import numpy as np
 import pytest
 
@@ -27,13 +27,12 @@ def _run(monkeypatch, cuda, n, nproj, nz, g, theta, env):
     return f.cpu().numpy()
 
 
-# the radices of 2n: 17 4 | 9 8 | 11 8 | 6 16 | 13 8 | 9 3 4 | 5 5 4 | 10 16 | 7 7 4 | 14 16 |
-# 18 16 | 15 4 16 .. | 15 6 16 | 15 3 16 4 | 17 18 16; a prime above 17 at 38 and 1058
+# fewer than 640 columns in all (within the grid); beside the 32 x 32 and 64 x 32
+# tiles; one, several and a remainder of pairs per block; primes of 2n up to 1223
 @pytest.mark.parametrize("n,nproj,nz", [
-    (34, 5, 3), (36, 7, 1), (44, 9, 2), (48, 5, 5), (52, 4, 1), (54, 6, 2), (50, 3, 4), (80, 5, 2),
-    (98, 4, 1), (112, 6, 3), (144, 5, 2), (240, 8, 2), (720, 6, 1), (1440, 5, 1), (2448, 6, 1),
-    (38, 5, 3), (1058, 5, 1)])
-def test_lines_vs_full_transform(cuda, monkeypatch, n, nproj, nz):
+    (34, 5, 3), (240, 8, 2), (319 * 2, 5, 1), (640, 4, 1), (38, 5, 20), (66, 3, 10), (98, 4, 8),
+    (300, 5, 40), (720, 6, 5), (1058, 5, 9), (2446, 3, 1), (2448, 6, 2)])
+def test_columns_vs_full_transform(cuda, monkeypatch, n, nproj, nz):
     import torch
     rng = np.random.default_rng(n)
     g = torch.as_tensor(rng.standard_normal((nz, nproj, n, 2)).astype(np.float32), device=cuda)
@@ -42,7 +41,17 @@ def test_lines_vs_full_transform(cuda, monkeypatch, n, nproj, nz):
     args = (monkeypatch, cuda, n, nproj, nz, g, theta)
     want = _run(*args, {"TCB_FOURIERREC_FULL_FFT2D": "1"})
     assert rel_l2(_run(*args, {}), want) < 1e-6
-    assert rel_l2(_run(*args, {"TCB_FOURIERREC_FFT": "cufft"}), want) < 1e-6
+
+
+@pytest.mark.parametrize("n,nz", [(128, 5), (256, 12)])
+def test_columns_of_power_of_two_widths(cuda, monkeypatch, n, nz):
+    """cuFFT's route where the library's own transform is the usual one."""
+    import torch
+    g = torch.randn((nz, 30, n, 2), generator=torch.Generator(device=cuda).manual_seed(n),
+                    device=cuda)
+    theta = torch.as_tensor((np.arange(30) * np.pi / 30 + 0.01).astype(np.float32), device=cuda)
+    args = (monkeypatch, cuda, n, 30, nz, g, theta)
+    assert rel_l2(_run(*args, {"TCB_FOURIERREC_FFT": "cufft"}), _run(*args, {})) < 1e-6
 
 
 def test_little_memory(cuda):

@@ -38,7 +38,6 @@
 #include <vector>
 
 #include "common.cuh"
-#include "fft_mixed.cuh"
 #include "fft_pow2.cuh"
 #include "tcgen05.cuh"
 
@@ -1417,22 +1416,21 @@ __global__ void deapod_terms(float4 *__restrict__ tab, int n) {
   tab[i] = make_float4(d, q, (float)sx, (float)sy);
 }
 
-// Deapodized value from the terms of column tx (X) and row ty (Y);
-// mun2 = mu * n^2, nsign = 1 - n % 4.
-__device__ __forceinline__ float2 deapod_terms_value(float2 v, const float4 X, const float4 Y,
-                                                     float mun2, int nproj, float nsign) {
-  const float sgn = X.z * Y.w;
-  v.x *= sgn;
-  v.y *= sgn;
+// What a value is deapodized by, from the terms of column tx (X) and row ty (Y):
+// the signed weight, and 1 inside the circle, 0 outside; mun2 = mu * n^2,
+// nsign = 1 - n % 4.
+__device__ __forceinline__ float2 deapod_factor(const float4 X, const float4 Y, float mun2,
+                                                int nproj, float nsign) {
   const float dx = X.x, dy = Y.x, x = X.y, y = Y.y;
   float phi = __expf(mun2 * (dx * dx + dy * dy)) / nproj;
   phi *= nsign;
-  v.x *= phi;
-  v.y *= phi;
-  const float lam = (float)((4 * x * x + 4 * y * y) < 1);
-  v.x *= lam;
-  v.y *= lam;
-  return v;
+  return make_float2(X.z * Y.w * phi, (float)((4 * x * x + 4 * y * y) < 1));
+}
+
+__device__ __forceinline__ float2 deapod_terms_value(float2 v, const float4 X, const float4 Y,
+                                                     float mun2, int nproj, float nsign) {
+  const float2 q = deapod_factor(X, Y, mun2, nproj, nsign);
+  return make_float2(v.x * q.x * q.y, v.y * q.x * q.y);
 }
 
 template <typename OutT>
@@ -1472,44 +1470,72 @@ __global__ void deapod_kernel(const float2 *__restrict__ grid, OutT *__restrict_
 // cuFFT's pruned inverse transform (2n not a power of two, or cuFFT forced): the
 // n kept columns of the row-transformed grid, transposed to t[z][c][y], so that
 // the column transforms run on contiguous lines (8 pairs at 2n = 4896: 2.2 ms
-// strided within the grid, 0.75 ms contiguous and 0.36 ms for this copy).
-// 32 x 32 tiles through shared memory.
+// strided within the grid, 0.53 ms contiguous and 0.26 ms for this copy, 0.33 ms
+// by 32 x 32 values).  Tiles of 64 rows x 32 columns through shared memory, eight
+// loads in flight per thread; HBM bounds it.
+constexpr int CT_ROWS = 64;
 __global__ void __launch_bounds__(256)
     crop_transpose(const float2 *__restrict__ grid, float2 *__restrict__ t, int n) {
-  __shared__ float2 tile[32][33];
+  __shared__ float2 tile[CT_ROWS][33];
   const int twon = 2 * n, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+  const int c0 = blockIdx.x * 32, y0 = blockIdx.y * CT_ROWS;
   const float2 *src = grid + (size_t)blockIdx.z * twon * twon + n / 2;
   float2 *dst = t + (size_t)blockIdx.z * n * twon;
-  for (int k = w; k < 32; k += 8)
-    if (y0 + k < twon && c0 + lane < n)
-      tile[k][lane] = src[(size_t)(y0 + k) * twon + c0 + lane];
+  if (c0 + lane < n)
+#pragma unroll
+    for (int k = 0; k < CT_ROWS; k += 8)
+      if (y0 + k + w < twon) tile[k + w][lane] = __ldcs(src + (size_t)(y0 + k + w) * twon + c0 + lane);
   __syncthreads();
-  for (int k = w; k < 32; k += 8)
-    if (c0 + k < n && y0 + lane < twon) dst[(size_t)(c0 + k) * twon + y0 + lane] = tile[lane][k];
+#pragma unroll
+  for (int k = 0; k < 32; k += 8)
+    if (c0 + k + w < n)
+#pragma unroll
+      for (int y = lane; y < CT_ROWS; y += 32)
+        if (y0 + y < twon) dst[(size_t)(c0 + k + w) * twon + y0 + y] = tile[y][k + w];
 }
 
-// deapod_kernel on the transposed columns t[z][c][y].
+// deapod_kernel on the transposed columns t[z][c][y]: a block takes a 32 x 32 tile
+// of `zper` pairs, so that a pixel's exponential and division serve them all, the
+// next pair's values in flight while one's are stored (8 pairs of 2448^2: 0.26 ->
+// 0.16 ms).
 template <typename OutT>
 __global__ void __launch_bounds__(256)
     deapod_transposed(const float2 *__restrict__ t, OutT *__restrict__ f,
-                      const float4 *__restrict__ dtab, Geom geo, int unpack) {
-  __shared__ float2 tile[32][33];
+                      const float4 *__restrict__ dtab, Geom geo, int unpack, int zper) {
+  __shared__ float2 tile[2][32][33];
   const int n = geo.n, twon = geo.twon, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, z = blockIdx.z;
-  const float2 *src = t + (size_t)z * n * twon + n / 2 + 1;
-  for (int k = w; k < 32; k += 8)
-    if (x0 + k < n && y0 + lane < n) tile[k][lane] = src[(size_t)(x0 + k) * twon + y0 + lane];
-  __syncthreads();
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
+  const int z0 = blockIdx.z * zper, z1 = min(geo.nz, z0 + zper);
   const int tx = x0 + lane;
-  if (tx >= n) return;
-  for (int k = w; k < 32; k += 8) {
-    const int ty = y0 + k;
-    if (ty < n)
-      store_out(f,
-                deapod_terms_value(tile[lane][k], __ldg(dtab + tx), __ldg(dtab + ty),
-                                   geo.mu * (n * n), geo.nproj, (float)(1 - n % 4)),
-                tx, ty, z, geo, unpack);
+  float2 q[4], v[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    q[j] = make_float2(0.f, 0.f);
+    if (tx < n && y0 + w + 8 * j < n)
+      q[j] = deapod_factor(__ldg(dtab + tx), __ldg(dtab + y0 + w + 8 * j), geo.mu * (n * n),
+                           geo.nproj, (float)(1 - n % 4));
+  }
+  auto load = [&](int z) {
+    const float2 *src = t + (size_t)z * n * twon + n / 2 + 1 + y0 + lane;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (x0 + w + 8 * j < n && y0 + lane < n) v[j] = __ldcs(src + (size_t)(x0 + w + 8 * j) * twon);
+  };
+  load(z0);
+  for (int z = z0; z < z1; z++) {
+    float2(&tl)[32][33] = tile[z & 1];
+#pragma unroll
+    for (int j = 0; j < 4; j++) tl[w + 8 * j][lane] = v[j];
+    if (z + 1 < z1) load(z + 1);
+    __syncthreads();
+    if (tx < n)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (y0 + w + 8 * j < n) {
+          const float2 u = tl[lane][w + 8 * j];
+          store_out(f, make_float2(u.x * q[j].x * q[j].y, u.y * q[j].x * q[j].y), tx,
+                    y0 + w + 8 * j, z, geo, unpack);
+        }
   }
 }
 
@@ -1787,9 +1813,6 @@ struct tcb_fourierrec {
   // transforms over only the n columns [n/2, 3n/2) that deapodization reads.
   cufftHandle plan_rows = 0, plan_cols = 0;
   bool pruned = false;
-  // the same two passes on the library's mixed-radix lines (mix.n = 2n, else 0)
-  tcb::mixfft::Plan mix;
-  float2 *mixtw = nullptr;
   // Own pruned FFT (rows pass, then columns pass fused with deapodization,
   // or the reverse) when 2n is a power of two in [256, 8192]: own_n = 2n,
   // else 0.
@@ -1853,8 +1876,6 @@ void fr_release(tcb_fourierrec *h) {
   cudaFree(h->grid);
   cudaFree(h->g32);
   cudaFree(h->t1);
-  cudaFree(h->mixtw);
-  h->mixtw = nullptr;
   cudaFree(h->tw);
   cudaFree(h->dtab);
   h->dtab = nullptr;
@@ -1938,7 +1959,7 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
     gc = h->g32;
   }
   TCB_CUFFT(cufftSetStream(h->plan1d, s));
-  if (h->own_n || h->mix.n) {
+  if (h->own_n) {
   } else if (h->pruned) {
     TCB_CUFFT(cufftSetStream(h->plan_rows, s));
     TCB_CUFFT(cufftSetStream(h->plan_cols, s));
@@ -2066,24 +2087,13 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
   }
   {
     StageTimer st("fr_fft2d", s);
-    if (h->mix.n) {
-      const size_t sm = mixfft::smem_bytes(h->mix.n);
-      const int lo = geo.n / 2, nt = h->mix.threads;
-      mixfft::ifft_lines<<<(unsigned)(2 * h->n * h->nz), nt, sm, s>>>(h->grid, h->mixtw, h->mix,
-                                                                      lo, lo + geo.n);
-      crop_transpose<<<dim3(ceil_div(h->n, 32), ceil_div(2 * h->n, 32), (unsigned)h->nz), 256, 0,
-                       s>>>(h->grid, h->t1, geo.n);
-      mixfft::ifft_lines<<<(unsigned)(h->n * h->nz), nt, sm, s>>>(h->t1, h->mixtw, h->mix, lo + 1,
-                                                                  lo + 1 + geo.n);
-      TCB_LAUNCH_CHECK();
-      count_launch(3);
-    } else if (h->pruned) {
+    if (h->pruned) {
       // separable: all rows along x, then the kept columns along y, per pair
       TCB_CUFFT(cufftExecC2C(h->plan_rows, (cufftComplex *)h->grid, (cufftComplex *)h->grid,
                              CUFFT_INVERSE));
       if (h->t1) {
-        crop_transpose<<<dim3(ceil_div(h->n, 32), ceil_div(2 * h->n, 32), (unsigned)h->nz), 256,
-                         0, s>>>(h->grid, h->t1, geo.n);
+        crop_transpose<<<dim3(ceil_div(h->n, 32), ceil_div(2 * h->n, CT_ROWS), (unsigned)h->nz),
+                         256, 0, s>>>(h->grid, h->t1, geo.n);
         TCB_LAUNCH_CHECK();
         count_launch();
         TCB_CUFFT(cufftExecC2C(h->plan_cols, (cufftComplex *)h->t1, (cufftComplex *)h->t1,
@@ -2103,11 +2113,16 @@ int fr_run(tcb_fourierrec *h, void *f, void *g, void *stream, int unpack) {
   {
     StageTimer st("fr_deapod", s);
     if (h->pruned && h->t1) {
-      const dim3 grd(ceil_div(h->n, 32), ceil_div(h->n, 32), (unsigned)h->nz);
+      // pairs per block: up to 8 that leave 8 blocks per SM
+      const size_t tiles = (size_t)ceil_div(h->n, 32) * ceil_div(h->n, 32) * h->nz;
+      const int zper = (int)std::min<size_t>({8, h->nz, std::max<size_t>(1, tiles / (8 * sm_count()))});
+      const dim3 grd(ceil_div(h->n, 32), ceil_div(h->n, 32), ceil_div(h->nz, zper));
       if (out_half)
-        deapod_transposed<__half><<<grd, 256, 0, s>>>(h->t1, (__half *)f, h->dtab, geo, unpack);
+        deapod_transposed<__half>
+            <<<grd, 256, 0, s>>>(h->t1, (__half *)f, h->dtab, geo, unpack, zper);
       else
-        deapod_transposed<float><<<grd, 256, 0, s>>>(h->t1, (float *)f, h->dtab, geo, unpack);
+        deapod_transposed<float>
+            <<<grd, 256, 0, s>>>(h->t1, (float *)f, h->dtab, geo, unpack, zper);
     } else {
       dim3 blk(32, 8), grd(ceil_div(h->n, 32), ceil_div(h->n, 8), (unsigned)h->nz);
       if (out_half)
@@ -2523,41 +2538,18 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
   }
   if (r == CUFFT_SUCCESS && !h->pruned)
     r = cufftPlanMany(&h->plan2d, 2, len2, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, (int)nz);
-  // the columns on a transposed copy, if that fits beside what has to
+  // The columns on a transposed copy, if that fits beside what has to, and for 640
+  // columns or more (of all pairs): the copy is one more launch (260 columns, one
+  // pair: the call 0.031 ms within the grid and 0.039 on the copy; 700 columns 0.056
+  // and 0.054, 4 pairs of 260 0.055 and 0.045).
   auto copy = [&]() {
+    if (n * nz < 640) return false;
     if (cudaMalloc(&h->t1, nz * n * N2 * sizeof(float2)) == cudaSuccess) return true;
     cudaGetLastError();
     h->t1 = nullptr;
     return false;
   };
-  auto no_copy = [&]() {
-    cudaGetLastError();
-    cudaFree(h->t1);
-    h->t1 = nullptr;
-  };
-  if (r == CUFFT_SUCCESS && h->pruned && !h->own_n && own_sel && N2 <= (size_t)mixfft::MAX_N) {
-    // 2n a product of primes up to 17 (8 pairs at 4896 =
-    // 17 18 16: 1.73 ms with the copy between the passes; cuFFT's passes 4.9)
-    std::vector<float2> twh;
-    const mixfft::Plan mix = mixfft::make_plan((int)N2, twh);
-    if (mix.n && copy()) {
-      if (cudaMalloc(&h->mixtw, twh.size() * sizeof(float2)) != cudaSuccess) {
-        h->mixtw = nullptr;
-        no_copy();
-      } else {
-        e = cudaMemcpy(h->mixtw, twh.data(), twh.size() * sizeof(float2), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-          e = cudaFuncSetAttribute(mixfft::ifft_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)mixfft::smem_bytes(mixfft::MAX_N));
-        if (e != cudaSuccess) {
-          set_error("tcb_fourierrec_create: FFT setup failed: %s", cudaGetErrorString(e));
-          return fail(TCB_ERR_CUDA);
-        }
-        h->mix = mix;
-      }
-    }
-  }
-  if (r == CUFFT_SUCCESS && h->pruned && !h->own_n && !h->mix.n) {
+  if (r == CUFFT_SUCCESS && h->pruned && !h->own_n) {
     int lr[1] = {(int)(2 * n)};
     r = cufftPlanMany(&h->plan_rows, 1, lr, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
                       (int)(2 * n * nz));
@@ -2565,7 +2557,9 @@ extern "C" int tcb_fourierrec_create(tcb_fourierrec **out, size_t nproj, size_t 
         cufftPlanMany(&h->plan_cols, 1, lr, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C,
                       (int)(n * nz)) != CUFFT_SUCCESS) {
       // no room for this plan's workspace beside the copy
-      no_copy();
+      cudaGetLastError();
+      cudaFree(h->t1);
+      h->t1 = nullptr;
       h->plan_cols = 0;
     }
     int emb[1] = {(int)(2 * n)};
