@@ -1416,21 +1416,22 @@ __global__ void deapod_terms(float4 *__restrict__ tab, int n) {
   tab[i] = make_float4(d, q, (float)sx, (float)sy);
 }
 
-// What a value is deapodized by, from the terms of column tx (X) and row ty (Y):
-// the signed weight, and 1 inside the circle, 0 outside; mun2 = mu * n^2,
-// nsign = 1 - n % 4.
-__device__ __forceinline__ float2 deapod_factor(const float4 X, const float4 Y, float mun2,
-                                                int nproj, float nsign) {
+// Deapodized value from the terms of column tx (X) and row ty (Y);
+// mun2 = mu * n^2, nsign = 1 - n % 4.
+__device__ __forceinline__ float2 deapod_terms_value(float2 v, const float4 X, const float4 Y,
+                                                     float mun2, int nproj, float nsign) {
+  const float sgn = X.z * Y.w;
+  v.x *= sgn;
+  v.y *= sgn;
   const float dx = X.x, dy = Y.x, x = X.y, y = Y.y;
   float phi = __expf(mun2 * (dx * dx + dy * dy)) / nproj;
   phi *= nsign;
-  return make_float2(X.z * Y.w * phi, (float)((4 * x * x + 4 * y * y) < 1));
-}
-
-__device__ __forceinline__ float2 deapod_terms_value(float2 v, const float4 X, const float4 Y,
-                                                     float mun2, int nproj, float nsign) {
-  const float2 q = deapod_factor(X, Y, mun2, nproj, nsign);
-  return make_float2(v.x * q.x * q.y, v.y * q.x * q.y);
+  v.x *= phi;
+  v.y *= phi;
+  const float lam = (float)((4 * x * x + 4 * y * y) < 1);
+  v.x *= lam;
+  v.y *= lam;
+  return v;
 }
 
 template <typename OutT>
@@ -1507,13 +1508,15 @@ __global__ void __launch_bounds__(256)
   const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
   const int z0 = blockIdx.z * zper, z1 = min(geo.nz, z0 + zper);
   const int tx = x0 + lane;
-  float2 q[4], v[4];
+  float q[4];  // signed weights, 0 outside the circle
+  float2 v[4];
 #pragma unroll
   for (int j = 0; j < 4; j++) {
-    q[j] = make_float2(0.f, 0.f);
+    q[j] = 0.f;
     if (tx < n && y0 + w + 8 * j < n)
-      q[j] = deapod_factor(__ldg(dtab + tx), __ldg(dtab + y0 + w + 8 * j), geo.mu * (n * n),
-                           geo.nproj, (float)(1 - n % 4));
+      q[j] = deapod_terms_value(make_float2(1.f, 0.f), __ldg(dtab + tx),
+                                __ldg(dtab + y0 + w + 8 * j), geo.mu * (n * n), geo.nproj,
+                                (float)(1 - n % 4)).x;
   }
   auto load = [&](int z) {
     const float2 *src = t + (size_t)z * n * twon + n / 2 + 1 + y0 + lane;
@@ -1533,8 +1536,7 @@ __global__ void __launch_bounds__(256)
       for (int j = 0; j < 4; j++)
         if (y0 + w + 8 * j < n) {
           const float2 u = tl[lane][w + 8 * j];
-          store_out(f, make_float2(u.x * q[j].x * q[j].y, u.y * q[j].x * q[j].y), tx,
-                    y0 + w + 8 * j, z, geo, unpack);
+          store_out(f, make_float2(u.x * q[j], u.y * q[j]), tx, y0 + w + 8 * j, z, geo, unpack);
         }
   }
 }
